@@ -10,6 +10,7 @@
 #include "engine.cuh"
 #include "layout.cuh"
 #include "mstep2d.cuh"
+#include "pair_transform.cuh"
 #include "resample.cuh"
 
 namespace binder {
@@ -224,6 +225,12 @@ void MStep::enqueue(const float *r, float *d, const float *xpos, const float *D,
                            s);
         a.noise = noise;
     }
+    // BF16 operands and axes of at most 256: two passes per launch, all components in one launch
+    if (bf16 && pair_supported(nx, ny, nz, planes)) {
+        a.chain_comps = chains > 1 ? ncomp : 0;
+        run_pairs(a, ncomp * chains, planes, s, r, d, xpos);
+        return;
+    }
     if (chains > 1) {
         // chains x components per launch: enough tiles to fill the GPU without stream branches
         a.chain_comps = ncomp;
@@ -244,6 +251,28 @@ void MStep::enqueue(const float *r, float *d, const float *xpos, const float *D,
     } else {
         run_chain(a, 0, ncomp, s, r, d, xpos, tc, planes);
     }
+}
+
+// the M-step of a volume as three launches of paired passes (an image's x passes as one), for nc
+// components on stream s
+void MStep::run_pairs(AxisArgs<float> a, int nc, int planes, cudaStream_t s, const float *r,
+                      float *d, const float *xpos) {
+    a.comp0 = 0;
+    if (nz == 1) {
+        a.in = r; a.out = t1; a.n = ny; a.outer = nx; a.s = 1;
+        launch_axis_pass_tc(a, dct.ufwd[1], nullptr, kEpiNone, nc, planes, s, false, true);
+        a.in = t1;
+        launch_pair_pass(a, kPairSpectral, nx, ny, nz, dct.ufwd[0], dct.uinv[0], nc, planes, s);
+        a.out = d; a.xpos = xpos;
+        launch_axis_pass_tc(a, dct.uinv[1], nullptr, kEpiPositions, nc, planes, s, false, true);
+        return;
+    }
+    a.in = r; a.out = t1;
+    launch_pair_pass(a, kPairForward, nx, ny, nz, dct.ufwd[2], dct.ufwd[1], nc, planes, s);
+    a.in = t1;
+    launch_pair_pass(a, kPairSpectral, nx, ny, nz, dct.ufwd[0], dct.uinv[0], nc, planes, s);
+    a.out = d; a.xpos = xpos;
+    launch_pair_pass(a, kPairInverse, nx, ny, nz, dct.uinv[1], dct.uinv[2], nc, planes, s);
 }
 
 // the pass sequence of one M-step for components [c0, c0 + nc) on stream s

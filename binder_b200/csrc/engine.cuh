@@ -53,6 +53,8 @@ struct MStep {
                  double rho_p, const double eta2[3], const int *skip, cudaStream_t s);
     void run_chain(AxisArgs<float> a, int c0, int nc, cudaStream_t s, const float *r, float *d,
                    const float *xpos, bool tc, int planes);
+    void run_pairs(AxisArgs<float> a, int nc, int planes, cudaStream_t s, const float *r, float *d,
+                   const float *xpos);
 };
 
 // A captured chunk of EM iterations, replayed by later EM calls while the parameters it was
