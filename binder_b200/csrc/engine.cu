@@ -402,7 +402,7 @@ Registration::~Registration() {
     const cudaStream_t s = own_stream_;
     dfree(d_, s); dfree(x_, s); dfree(r_, s); dfree(D_, s); dfree(theta_, s); dfree(hist_, s);
     dfree(hcnt_, s); dfree(u_, s); dfree(vpad_, s); dfree(mean_, s);
-    dfree(m2_, s); dfree(hfix_, s); dfree(mpart_, s); dfree(hdone_, s);
+    dfree(m2_, s); dfree(hfix_, s); dfree(mpart_, s);
     dfree(stats_, s); dfree(st_, s); dfree(d0_, s); dfree(theta0_, s);
     dfree(ssd_, s); dfree(ssd0_, s); dfree(colmax_, s); dfree(colmax0_, s);
     dfree(fx_, s); dfree(fn_, s); dfree(fst_, s); dfree(fst0_, s); dfree(fstats_, s);
@@ -471,7 +471,7 @@ void Registration::load_bins(double alpha, const float *theta, int K, int L, int
     const long nv = V_ + M - 1, nn = Vn_ + M - 1;  // bins read: [index + m], m < M
     const long cells = (long)M * K * L;
     dfree(u_, s); dfree(vpad_, s); dfree(theta_, s); dfree(hist_, s);
-    dfree(hcnt_, s); dfree(hfix_, s); dfree(mpart_, s); dfree(hdone_, s);
+    dfree(hcnt_, s); dfree(hfix_, s); dfree(mpart_, s);
     dfree(theta0_, s);
     u_ = dalloc<uint8_t>((size_t)nv, s);
     theta0_ = dalloc<float>((size_t)cells, s);
@@ -497,10 +497,9 @@ void Registration::load_bins(double alpha, const float *theta, int K, int L, int
     // channel, K <= 64)
     if (M == 1 && K <= 64) {
         hfix_ = dalloc<unsigned long long>((size_t)K * L, s);
-        mpart_ = dalloc<double>(kMaxEmCtas, s);
-        hdone_ = dalloc<unsigned>(1, s);
+        mpart_ = dalloc<double>(kEmPartials, s);
+        BINDER_CUDA(cudaMemsetAsync(mpart_, 0, sizeof(double) * kEmPartials, s));
         BINDER_CUDA(cudaMemsetAsync(hfix_, 0, sizeof(unsigned long long) * K * L, s));
-        BINDER_CUDA(cudaMemsetAsync(hdone_, 0, sizeof(unsigned), s));
     }
     BINDER_CUDA(cudaMemcpyAsync(theta_, theta, sizeof(float) * cells, cudaMemcpyDefault, s));
     BINDER_CUDA(cudaMemcpyAsync(theta0_, theta_, sizeof(float) * cells, cudaMemcpyDeviceToDevice, s));
@@ -563,7 +562,7 @@ void Registration::set_ssd_likelihood(int bins, double sigma2, int shift_scale, 
     h.shift_scale = shift_scale ? 1 : 0;
     BINDER_CUDA(cudaMemcpyAsync(ssd_, &h, sizeof h, cudaMemcpyHostToDevice, s));
     BINDER_CUDA(cudaMemcpyAsync(ssd0_, &h, sizeof h, cudaMemcpyHostToDevice, s));
-    launch_ssd_update(theta_, colmax_, nullptr, bins, bins, 0, ssd_, nullptr, s);
+    launch_ssd_update(theta_, colmax_, nullptr, nullptr, nullptr, bins, bins, 0, ssd_, nullptr, s);
     BINDER_CUDA(cudaMemcpyAsync(theta0_, theta_, sizeof(float) * bins * bins,
                                 cudaMemcpyDeviceToDevice, s));
     BINDER_CUDA(cudaMemcpyAsync(colmax0_, colmax_, sizeof(float) * bins, cudaMemcpyDeviceToDevice,
@@ -703,7 +702,7 @@ EStepArgs Registration::estep_args(const int *skip) const {
     const View w = estep_view();
     EStepArgs e{};
     e.d = d_; e.r = r_; e.x = x_; e.u = u_; e.vpad = vpad_; e.theta = theta_; e.hist = hist_;
-    e.hfix = hfix_; e.mpart = mpart_; e.hdone = hdone_;
+    e.hfix = hfix_; e.mpart = mpart_;
     e.hcnt = hcnt_; e.st = st_; e.skip = skip; e.V = V_;
     e.nx = w.nx; e.ny = w.ny; e.nz = w.nz; e.nxn = w.nxn; e.nyn = w.nyn; e.nzn = w.nzn;
     e.P = P_; e.PZ = PZ_; e.pyn = pyn_; e.zp = zp_; e.K = K_; e.L = L_; e.dim = N_;
@@ -723,11 +722,13 @@ void Registration::enqueue_em_iteration(int max_iter, double th, int update, cud
     BINDER_CUDA(cudaEventRecord(lk_fork_, s));
     BINDER_CUDA(cudaStreamWaitEvent(lk_stream_, lk_fork_, 0));
     if (lk_ == 1)
-        launch_ssd_update(theta_, colmax_, hist_, K_, L_, update, ssd_, st_, lk_stream_);
+        launch_ssd_update(theta_, colmax_, hist_, hfix_, mpart_, K_, L_, update, ssd_, st_,
+                          lk_stream_);
     else if (lk_ == 3)
         launch_ssdf_update(fst_, fstats_, update, st_, lk_stream_);
     else
-        launch_theta_update(theta_, hist_, M_ * K_, L_, alpha_, update, st_, lk_stream_);
+        launch_theta_update(theta_, hist_, lk_ == 2 ? nullptr : hfix_, mpart_, M_ * K_, L_, alpha_,
+                            update, st_, lk_stream_);
     BINDER_CUDA(cudaEventRecord(lk_join_, lk_stream_));
     const double eta2[3] = {eta_[0] * eta_[0], eta_[1] * eta_[1], eta_[2] * eta_[2]};
     mstep_.enqueue(r_, d_, x_, D_, st_, sigma2_, 0, 0, 1, seed_, chain_,
@@ -1117,10 +1118,12 @@ double Registration::profile_stage(int stage, int n) {
             mstep_.enqueue(r_, d_, x_, D_, st_, sigma2_, 0, 0, 1, seed_, chain_,
                            rho_[0] * rho_[1] * rho_[2], eta2, nullptr, stream_);
         else if (lk_ == 1)
-            launch_ssd_update(theta_, colmax_, hist_, K_, L_, 0, ssd_, st_, stream_);
+            launch_ssd_update(theta_, colmax_, hist_, hfix_, mpart_, K_, L_, 0, ssd_, st_, stream_);
         else if (lk_ == 3)
             launch_ssdf_update(fst_, fstats_, 0, st_, stream_);
-        else launch_theta_update(theta_, hist_, M_ * K_, L_, alpha_, 1, st_, stream_);
+        else
+            launch_theta_update(theta_, hist_, lk_ == 2 ? nullptr : hfix_, mpart_, M_ * K_, L_,
+                                alpha_, 1, st_, stream_);
     };
     one();  // warm-up
     cudaEvent_t t0, t1;
@@ -1135,6 +1138,8 @@ double Registration::profile_stage(int stage, int n) {
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
     BINDER_CUDA(cudaMemsetAsync(hist_, 0, sizeof(float) * M_ * K_ * L_, stream_));
+    if (hfix_)
+        BINDER_CUDA(cudaMemsetAsync(hfix_, 0, sizeof(unsigned long long) * K_ * L_, stream_));
     BINDER_CUDA(cudaStreamSynchronize(stream_));
     return ms / n;
 }

@@ -69,14 +69,19 @@ __device__ __forceinline__ void gather_bins(const EStepArgs &a, int ix, int iy, 
                       (DIM == 2 || ((iy - 1 + a.P >= 0) && (iy + 2 + a.P < a.nyn + 2 * a.P))) &&
                       (zz0 >= 0) && ((zz0 >> 2) + 2 <= (a.zp >> 2));
     if (fast) {
-        const int w = zz0 >> 2, sh = (zz0 & 3) * 8;
+        // one 64-bit base and word strides: 335 -> 326 us at 160x192x160 against a 64-bit product
+        // per row
+        const int sh = (zz0 & 3) * 8;
+        const unsigned sy = (unsigned)a.zp >> 2, sx = sy * (unsigned)a.pyn;  // words (zp % 4 == 0)
+        const uint32_t *base =
+            reinterpret_cast<const uint32_t *>(
+                a.vpad + ((long)(ix - 1 + a.P) * a.pyn + (y0 + Py)) * a.zp) + (zz0 >> 2);
 #pragma unroll
         for (int p = 0; p < 4; ++p)
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
-                const uint32_t *row = reinterpret_cast<const uint32_t *>(
-                    a.vpad + ((long)(ix - 1 + p + a.P) * a.pyn + (y0 + q + Py)) * a.zp);
-                const uint32_t lo = __ldg(row + w), hi = __ldg(row + w + 1);
+                const uint32_t *row = base + (p * sx + q * sy);
+                const uint32_t lo = __ldg(row), hi = __ldg(row + 1);
                 pk[p * Q + q] = __funnelshift_r(lo, hi, sh);
             }
     } else {
@@ -189,11 +194,17 @@ template <int TPB>
 __device__ __forceinline__ __half *half_slot(__half *col, int k) {
     return col + k * TPB;
 }
-// masses w.x, w.y of two neighbours with bins ka, kb (one FP32 to FP16 pair conversion)
+// masses w.x, w.y of two neighbours with bins ka, kb, added one after the other (one FP32 to FP16
+// pair conversion); the FP32 form loads both sums before either store, which halves the chain of
+// dependent shared-memory round trips (340 -> 335 us at 160x192x160; four at a time, with their
+// six comparisons, 345)
 template <int TPB>
 __device__ __forceinline__ void col_add2(float *__restrict__ col, int ka, int kb, float2 w) {
-    col[ka * TPB] += w.x;
-    col[kb * TPB] += w.y;
+    const float a = col[ka * TPB], b = col[kb * TPB];
+    const float na = a + w.x;
+    const float nb = (ka == kb ? na : b) + w.y;
+    col[ka * TPB] = na;
+    col[kb * TPB] = nb;
 }
 template <int TPB>
 __device__ __forceinline__ void col_add2(__half *__restrict__ col, int ka, int kb, float2 w) {
@@ -234,6 +245,9 @@ __device__ __forceinline__ void em_accumulate(const float *__restrict__ thu,
     float2 x01 = a01, x23 = a01;                    // sum of (p - 1) w
     float2 y01 = a01, y23 = a01;                    // sum of (q - 1) w
     int lo = 255, hi = 0;
+    // theta's address of byte c: one dot-product instruction instead of an extraction and an add
+    // (E-step 326 -> 319 us at 160x192x160); loads without memory clobber, theta is constant here
+    const unsigned tha = (unsigned)__cvta_generic_to_shared(thu);
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
@@ -244,8 +258,13 @@ __device__ __forceinline__ void em_accumulate(const float *__restrict__ thu,
             const uint32_t word = pk[p * Q + q];
             const int k0 = word & 0xff, k1 = (word >> 8) & 0xff, k2 = (word >> 16) & 0xff,
                       k3 = word >> 24;
-            const float2 w01 = __fmul2_rn(b01, make_float2(thu[k0], thu[k1]));
-            const float2 w23 = __fmul2_rn(b23, make_float2(thu[k2], thu[k3]));
+            float t0, t1, t2, t3;
+            asm("ld.shared.f32 %0, [%1];" : "=f"(t0) : "r"(__dp4a(word, 0x4u, tha)));
+            asm("ld.shared.f32 %0, [%1];" : "=f"(t1) : "r"(__dp4a(word, 0x400u, tha)));
+            asm("ld.shared.f32 %0, [%1];" : "=f"(t2) : "r"(__dp4a(word, 0x40000u, tha)));
+            asm("ld.shared.f32 %0, [%1];" : "=f"(t3) : "r"(__dp4a(word, 0x4000000u, tha)));
+            const float2 w01 = __fmul2_rn(b01, make_float2(t0, t1));
+            const float2 w23 = __fmul2_rn(b23, make_float2(t2, t3));
             col_add2<TPB>(col, k0, k1, w01);
             col_add2<TPB>(col, k2, k3, w23);
             a01 = __fadd2_rn(a01, w01);
@@ -362,15 +381,17 @@ __global__ void __launch_bounds__(TPB, HC ? 3 : (TPB > kFastThreads ? 1 : 2))
     float *thT = sm;                                             // [L][KP]
     unsigned *hs = reinterpret_cast<unsigned *>(sm + L * KP);    // [K][LP] CTA histogram (fixed)
     float *hkw = sm + L * KP + K * LP;  // per-thread bin masses: [K][TPB] FP32 or FP16
-    const int hk_words = HC ? ((K + 1) / 2) * TPB : K * TPB;
+    const int K4 = (K + 3) & ~3;  // rows of the columns
+    const int hk_words = HC ? (K4 / 2) * TPB : K4 * TPB;
     float *cmx = hkw + hk_words;                                 // [L] log-space column maxima
     __shared__ double red[32];
     if (LOGT)
         for (int l = threadIdx.x; l < L; l += TPB) cmx[l] = a.colmax[l];
     const float tscale = HC ? kHalfColScale : 1.0f;
+#pragma unroll 4
     for (int q = threadIdx.x; q < KL; q += TPB) {
         const int k = q / L, l = q - k * L;
-        thT[l * KP + k] = a.theta[q] * tscale;
+        thT[l * KP + k] = __ldg(a.theta + q) * tscale;
         hs[k * LP + l] = 0u;
     }
     for (int q = threadIdx.x; q < hk_words; q += TPB) hkw[q] = 0.0f;
@@ -408,11 +429,18 @@ __global__ void __launch_bounds__(TPB, HC ? 3 : (TPB > kFastThreads ? 1 : 2))
         const float inv = ok ? 1.0f / S : 0.0f;
         const float invs = inv * a.hscale;
         unsigned *hcol = hs + ui;  // hcol[k * LP]
-        for (int k = kmin; k <= kmax; ++k) {
-            const float m = col_get<TPB>(my, k);
-            if (m != 0.0f) {
-                if (ok) atomicAdd(&hcol[k * LP], __float2uint_rn(m * invs));
-                col_clear<TPB>(my, k);
+        // four bins at a time, their loads and conversions in flight together (the columns have a
+        // multiple of four rows; rows past K stay zero): one bin at a time, each waiting for the
+        // one before, the launch took 364 us instead of 340 at 160x192x160, 39 instead of 35 at 64^3
+        for (int k = kmin & ~3; k <= kmax; k += 4) {
+            float m[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) m[e] = col_get<TPB>(my, k + e);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (ok && m[e] != 0.0f)
+                    atomicAdd(&hcol[(k + e) * LP], __float2uint_rn(m[e] * invs));
+                col_clear<TPB>(my, k + e);
             }
         }
         if (!ok) {
@@ -439,37 +467,39 @@ __global__ void __launch_bounds__(TPB, HC ? 3 : (TPB > kFastThreads ? 1 : 2))
         return;
     }
     // Order-independent merge, so that EM is bitwise repeatable: the CTA histograms are integers
-    // and their 64-bit global sums are exact whatever order the CTAs arrive in; the last CTA to
-    // finish converts the sums to the FP32 histogram (one rounding per cell) and adds the CTAs'
-    // log-likelihood partials in CTA order.
+    // and their 64-bit global sums are exact whatever order the CTAs arrive in.  The likelihood
+    // update that follows on the stream converts the sums (one rounding per cell), clears them and
+    // adds the CTAs' log-likelihood partials in CTA order (merged_cell, merge_mll).  Done here by
+    // the last CTA to finish, it held up the M-step by 13 us whatever the volume.
     for (int q = threadIdx.x; q < KL; q += TPB) {
         const int k = q / L;
         const unsigned v = hs[k * LP + (q - k * L)];
         if (v) atomicAdd(&a.hfix[q], (unsigned long long)v);
     }
-    if (threadIdx.x == 0) a.mpart[blockIdx.x] = m;
-    __threadfence();
-    __syncthreads();
-    __shared__ unsigned last;
-    if (threadIdx.x == 0) last = atomicAdd(a.hdone, 1u) == gridDim.x - 1 ? 1u : 0u;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const double hinv = a.hinv;
-    for (int q = threadIdx.x; q < KL; q += TPB) {
-        const unsigned long long v = __ldcg(a.hfix + q);
-        if (v) {
-            a.hist[q] += (float)((double)v * hinv);
-            a.hfix[q] = 0ull;
+    if (threadIdx.x == 0) {
+        a.mpart[blockIdx.x] = m;
+        if (blockIdx.x == 0) {
+            a.mpart[kMaxEmCtas] = a.hinv;
+            a.mpart[kMaxEmCtas + 1] = (double)gridDim.x;
         }
     }
+}
+
+// Cell q of the joint histogram for the likelihood update: the FP32 histogram, plus what the
+// single-pass E-step left in the 64-bit sums (EStepArgs::hfix) at the scale it left in mpart.
+__device__ __forceinline__ float merged_cell(const float *hist, const unsigned long long *hfix,
+                                             double hinv, int q) {
+    const float h = hist[q];
+    return hfix ? h + (float)((double)hfix[q] * hinv) : h;
+}
+
+// the CTAs' log-likelihood partials in CTA order into st->mll; every thread of the block
+__device__ __forceinline__ void merge_mll(const double *mpart, DevState *st, double *red) {
+    const unsigned n = (unsigned)mpart[kMaxEmCtas + 1];
     double part = 0.0;
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += TPB) part += __ldcg(a.mpart + b);
+    for (unsigned b = threadIdx.x; b < n; b += blockDim.x) part += mpart[b];
     const double tot = block_sum(part, red);
-    if (threadIdx.x == 0) {
-        a.st->mll += tot;
-        *a.hdone = 0u;
-    }
+    if (threadIdx.x == 0) st->mll += tot;
 }
 
 // EM E-step with the MI filter likelihood (BINDER/src/cpu/MILikelihoodFilter.cpp:53-68 and
@@ -1269,12 +1299,16 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
     if (threadIdx.x == 0 && dg > 0.0) atomicAdd(&st->degenerate, (unsigned long long)dg);
 }
 
-// MILikelihood.cpp:71-86 (update) and :33-39, :183-206 (cost), one CTA
-__global__ void theta_update_kernel(float *theta, float *hist, int K, int L, double alpha,
-                                    int update, DevState *st) {
+// MILikelihood.cpp:71-86 (update) and :33-39, :183-206 (cost), one CTA; the E-step's sums (hfix,
+// mpart, or null) merged into the histogram it reads
+__global__ void theta_update_kernel(float *theta, float *hist, unsigned long long *hfix,
+                                    const double *mpart, int K, int L, double alpha, int update,
+                                    DevState *st) {
     if (st->done) return;
-    __shared__ double rowlp[32];
+    __shared__ double rowlp[32], red[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const double hinv = hfix ? mpart[kMaxEmCtas] : 0.0;
+    if (hfix) merge_mll(mpart, st, red);
     double lp_total = 0.0;
     // the log-normaliser terms are the same for every row: lgamma(sum alpha) - L lgamma(alpha)
     double sum_alpha = 0.0;
@@ -1285,10 +1319,12 @@ __global__ void theta_update_kernel(float *theta, float *hist, int K, int L, dou
     for (int k = wid; k < K; k += nw) {
         if (update) {
             double s = 0.0;
-            for (int l = lane; l < L; l += 32) s += (double)hist[k * L + l] + alpha - 1.0;
+            for (int l = lane; l < L; l += 32)
+                s += (double)merged_cell(hist, hfix, hinv, k * L + l) + alpha - 1.0;
             s = warp_sum(s);
             for (int l = lane; l < L; l += 32)
-                theta[k * L + l] = (float)(((double)hist[k * L + l] + alpha - 1.0) / s);
+                theta[k * L + l] =
+                    (float)(((double)merged_cell(hist, hfix, hinv, k * L + l) + alpha - 1.0) / s);
             __syncwarp();
         }
         double sl = 0.0;
@@ -1297,7 +1333,10 @@ __global__ void theta_update_kernel(float *theta, float *hist, int K, int L, dou
         if (lane == 0) lp_total += -(lnorm + sl);
     }
     __syncthreads();  // every row has been read before the histogram is cleared
-    for (int q = threadIdx.x; q < K * L; q += blockDim.x) hist[q] = 0.0f;
+    for (int q = threadIdx.x; q < K * L; q += blockDim.x) {
+        hist[q] = 0.0f;
+        if (hfix) hfix[q] = 0ull;
+    }
     if (lane == 0) rowlp[wid] = lp_total;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1454,7 +1493,8 @@ namespace {
 size_t fast_smem(int K, int L, int tpb, bool logt, bool half) {
     const bool w = tpb > kFastThreads;
     const int KP = w ? wide_pitch(K) : theta_pitch(K), LP = w ? wide_pitch(L) : theta_pitch(L);
-    return (size_t)(L * KP + K * LP + (half ? ((K + 1) / 2) * tpb : K * tpb) + (logt ? L : 0)) *
+    const int K4 = (K + 3) & ~3;
+    return (size_t)(L * KP + K * LP + (half ? K4 / 2 * tpb : K4 * tpb) + (logt ? L : 0)) *
            sizeof(float);
 }
 
@@ -1724,9 +1764,10 @@ void launch_estep(const EStepArgs &args, bool sample, int grid, cudaStream_t s, 
     BINDER_CUDA(cudaGetLastError());
 }
 
-void launch_theta_update(float *theta, float *hist, int K, int L, double alpha, int update,
-                         DevState *st, cudaStream_t s) {
-    count_launch(), theta_update_kernel<<<1, 1024, 0, s>>>(theta, hist, K, L, alpha, update, st);
+void launch_theta_update(float *theta, float *hist, unsigned long long *hfix, const double *mpart,
+                         int K, int L, double alpha, int update, DevState *st, cudaStream_t s) {
+    count_launch(), theta_update_kernel<<<1, 1024, 0, s>>>(theta, hist, hfix, mpart, K, L, alpha,
+                                                           update, st);
     BINDER_CUDA(cudaGetLastError());
 }
 
@@ -1739,9 +1780,13 @@ __device__ __forceinline__ double ssd_loglik(int k, int l, const SsdState &p) {
     return (adj * adj) / (-2.0 * p.sigma2) - log(sqrt(2.0 * 3.14159265358979323846 * p.sigma2));
 }
 
-__global__ void ssd_update_kernel(float *table, float *colmax, float *hist, int K, int L,
+__global__ void ssd_update_kernel(float *table, float *colmax, float *hist,
+                                  unsigned long long *hfix, const double *mpart, int K, int L,
                                   int update, SsdState *ps, DevState *st) {
     if (st && st->done) return;
+    __shared__ double red[32];
+    const double hinv = hfix ? mpart[kMaxEmCtas] : 0.0;
+    if (hfix) merge_mll(mpart, st, red);
     __shared__ double G[kLogMaxBins], S1[kLogMaxBins], S2[kLogMaxBins], D2[kLogMaxBins];
     __shared__ SsdState p;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1753,7 +1798,8 @@ __global__ void ssd_update_kernel(float *table, float *colmax, float *hist, int 
         for (int k = wid; k < K; k += nw) {
             double g = 0.0, s1 = 0.0, s2 = 0.0, d2 = 0.0;
             for (int l = lane; l < L; l += 32) {
-                const double h = (double)hist[k * L + l], df = (double)l - (double)k;
+                const double h = (double)merged_cell(hist, hfix, hinv, k * L + l),
+                             df = (double)l - (double)k;
                 g += h;
                 s1 += h * (double)l;
                 s2 += h * (double)l * (double)l;
@@ -1820,7 +1866,10 @@ __global__ void ssd_update_kernel(float *table, float *colmax, float *hist, int 
     }
     if (st && hist) {
         __syncthreads();  // every row was read before the histogram is cleared
-        for (int q = threadIdx.x; q < K * L; q += blockDim.x) hist[q] = 0.0f;
+        for (int q = threadIdx.x; q < K * L; q += blockDim.x) {
+            hist[q] = 0.0f;
+            if (hfix) hfix[q] = 0ull;
+        }
     }
 }
 
@@ -1918,10 +1967,12 @@ __global__ void ssd_sample_kernel(float *table, float *colmax, unsigned *hcnt, i
 }
 }  // namespace
 
-void launch_ssd_update(float *table, float *colmax, float *hist, int K, int L, int update,
-                       SsdState *p, DevState *st, cudaStream_t s) {
+void launch_ssd_update(float *table, float *colmax, float *hist, unsigned long long *hfix,
+                       const double *mpart, int K, int L, int update, SsdState *p, DevState *st,
+                       cudaStream_t s) {
     BINDER_CHECK(K >= 1 && K <= kLogMaxBins && L >= 1, "SSD bins must be in [1, 64]");
-    count_launch(), ssd_update_kernel<<<1, 256, 0, s>>>(table, colmax, hist, K, L, update, p, st);
+    count_launch(), ssd_update_kernel<<<1, 256, 0, s>>>(table, colmax, hist, hfix, mpart, K, L,
+                                                       update, p, st);
     BINDER_CUDA(cudaGetLastError());
 }
 

@@ -17,12 +17,11 @@ struct EStepArgs {
     const uint8_t *vpad;  // moving-image bins, zero-padded [nxn+2P][nyn+2P][zp bytes]
     const float *theta;   // [K*L]
     float *hist;          // EM: soft joint histogram [K*L] (accumulated)
-    // the single-pass EM kernel's order-independent merge (all three null: FP32 atomics instead):
-    // 64-bit fixed-point sums [K*L] (zero between launches), one log-likelihood partial per CTA
-    // [kMaxEmCtas], and the count of CTAs done (zero between launches)
+    // the single-pass EM kernel's order-independent merge (both null: FP32 atomics instead): 64-bit
+    // fixed-point sums [K*L], and one log-likelihood partial per CTA [kMaxEmCtas] followed by the
+    // sums' scale and the number of CTAs; the likelihood update that follows reads and clears them
     unsigned long long *hfix;
     double *mpart;
-    unsigned *hdone;
     unsigned *hcnt;       // Gibbs: joint counts [K*L] (accumulated)
     DevState *st;
     const int *skip;
@@ -64,6 +63,7 @@ struct EStepArgs {
 
 // CTAs of the single-pass EM kernel at most when it merges in fixed order (EStepArgs::mpart)
 constexpr int kMaxEmCtas = 2048;
+constexpr int kEmPartials = kMaxEmCtas + 2;  // doubles in EStepArgs::mpart
 // chains > 1: a batch of chains, the sampling E-step only (chain = blockIdx.y; buffers
 // [chains][dim][V] positions / dream locations, [chains][K][L] theta / counts, [chains] states)
 void launch_estep(const EStepArgs &a, bool sample, int grid, cudaStream_t s, int chains = 1);
@@ -121,8 +121,9 @@ struct SsdState {
 // of sigma^2 into st->lp_lik (:314-326), the log2 likelihood table [K][L] (normalised per column)
 // and its column maxima rebuilt from the parameters, and the histogram cleared.  st may be null
 // (table only, no histogram).  One CTA.
-void launch_ssd_update(float *table, float *colmax, float *hist, int K, int L, int update,
-                       SsdState *p, DevState *st, cudaStream_t s);
+void launch_ssd_update(float *table, float *colmax, float *hist, unsigned long long *hfix,
+                       const double *mpart, int K, int L, int update, SsdState *p, DevState *st,
+                       cudaStream_t s);
 
 // the sampler's draw of the SSD likelihood's parameters (SSDLikelihood.cpp:284-302) from the
 // sweep's counts hcnt [K][L] (Philox ctr {0, st->sweep, 6 / 7, chain}), the log2 table and its
@@ -131,9 +132,10 @@ void launch_ssd_sample(float *table, float *colmax, unsigned *hcnt, int K, int L
                        DevState *st, uint64_t seed, uint32_t chain, cudaStream_t s);
 
 // theta <- (hist + alpha - 1)/rowsum (if update), Dirichlet prior cost into st->lp_lik,
-// hist zeroed for the next iteration.  One CTA.
-void launch_theta_update(float *theta, float *hist, int K, int L, double alpha, int update,
-                         DevState *st, cudaStream_t s);
+// hist zeroed for the next iteration.  One CTA.  hfix / mpart: the single-pass E-step's sums and
+// partials (EStepArgs; null where it does not run), merged into hist and st->mll here.
+void launch_theta_update(float *theta, float *hist, unsigned long long *hfix, const double *mpart,
+                         int K, int L, double alpha, int update, DevState *st, cudaStream_t s);
 // theta_k ~ Dirichlet(counts_k + alpha) with Philox gammas (tag 4, sweep = st->sweep); counts zeroed
 void launch_dirichlet_sample(float *theta, unsigned *hcnt, int K, int L, double alpha,
                              uint64_t seed, uint32_t chain, DevState *st, cudaStream_t s,
