@@ -2,6 +2,7 @@
 // gamma-prior sampling, EM bookkeeping and FP64 Welford moments.
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 
@@ -1119,13 +1120,14 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
     const uint32_t chain = SAMPLE ? a.chain + blockIdx.y : a.chain;
     extern __shared__ __align__(16) float sm[];
     const int KL = a.K * a.L;
-    float *th = sm;
-    float *hs = sm + KL;                                 // EM histogram
-    unsigned *hc = reinterpret_cast<unsigned *>(sm + KL);  // Gibbs counts
-    float *cps = sm + 2 * KL + threadIdx.x;  // Gibbs: cdf at the end of node row r, cps[r * kEThreads]
+    float *cps = sm + threadIdx.x;  // Gibbs: cdf at the end of node row r, cps[r * kEThreads]
+    float *hs = sm + (SAMPLE ? 16 * kEThreads : 0);       // EM histogram
+    unsigned *hc = reinterpret_cast<unsigned *>(hs);      // Gibbs counts
+    float *th = hs + KL;  // theta transposed, [L][a.tpitch]
     __shared__ double red[32];
     for (int q = threadIdx.x; q < KL; q += blockDim.x) {
-        th[q] = a.theta[ks + q];
+        const int k = q / a.L;
+        th[(q - k * a.L) * a.tpitch + k] = a.theta[ks + q];
         if (SAMPLE) hc[q] = 0u; else hs[q] = 0.0f;
     }
     __syncthreads();
@@ -1149,8 +1151,16 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
         const float fx = (float)ix, fy = (float)iy, fz = (float)iz;
         uint32_t pk[R];
         gather_bins<DIM>(a, ix, iy, iz, pk);
-        const float *thc = th + a.u[i];  // theta column of this voxel's bin: thc[k * L]
+        const int ui = a.u[i];
+        const float *thc = th + ui * a.tpitch;  // theta of this voxel's bin: thc[k]
         const int L = a.L;
+        // theta of node c of a packed word, its address by one dot-product instruction
+        const unsigned tha = (unsigned)__cvta_generic_to_shared(thc);
+        auto theta_at = [&](uint32_t word, int c) {
+            float t;
+            asm("ld.shared.f32 %0, [%1];" : "=f"(t) : "r"(__dp4a(word, 4u << (8 * c), tha)));
+            return t;
+        };
         // LOGT (the SSD likelihood, sampling): thc holds log2 likelihoods, the spline weights
         // enter as log2 (-inf for a zero tap) and every neighbour's weight is exp2 of its term
         // minus the voxel's largest term (Registration.cpp:331-470)
@@ -1171,7 +1181,7 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
                         lm = fmaxf(lm, __fadd_rn(__fadd_rn(__fadd_rn(lx[p], ly[q]), lz[c]),
-                                                 thc[((word >> (8 * c)) & 0xff) * L]));
+                                                 theta_at(word, c)));
                 }
         }
 
@@ -1183,13 +1193,23 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
             for (int q = 0; q < Q; ++q) {
                 const float bxy = DIM == 3 ? __fmul_rn(bx[p], by[q]) : bx[p];
                 const uint32_t word = pk[p * Q + q];
+                float t4[4], w4[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) t4[c] = theta_at(word, c);
+                if (!LOGT) {
+                    const float2 bb = make_float2(bxy, bxy);
+                    const float2 w01 = __fmul2_rn(__fmul2_rn(bb, make_float2(bz[0], bz[1])),
+                                                  make_float2(t4[0], t4[1]));
+                    const float2 w23 = __fmul2_rn(__fmul2_rn(bb, make_float2(bz[2], bz[3])),
+                                                  make_float2(t4[2], t4[3]));
+                    w4[0] = w01.x; w4[1] = w01.y; w4[2] = w23.x; w4[3] = w23.y;
+                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const int k = (word >> (8 * c)) & 0xff;
                     const float w =
                         LOGT ? exp2f(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(lx[p], ly[q]),
-                                                                   lz[c]), thc[k * L]), -lm))
-                             : __fmul_rn(__fmul_rn(bxy, bz[c]), thc[k * L]);
+                                                                   lz[c]), t4[c]), -lm))
+                             : w4[c];
                     S = __fadd_rn(S, w);
                     Sx = fmaf((float)(p - 1), w, Sx);
                     if (DIM == 3) Sy = fmaf((float)(q - 1), w, Sy);
@@ -1208,7 +1228,6 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
             vp.store_r(a, i, V, fx + Sx * inv, fy + Sy * inv, fz + Sz * inv, cs);
             // pass 2: normalised posteriors into the histogram column u_i, runs of equal bins
             // combined in a register before each shared-memory atomic
-            const int ui = a.u[i];
             int ck = -1;
             float cacc = 0.0f;
 #pragma unroll
@@ -1220,7 +1239,7 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const int k = (word >> (8 * c)) & 0xff;
-                        const float w = __fmul_rn(__fmul_rn(bxy, bz[c]), thc[k * L]) * inv;
+                        const float w = __fmul_rn(__fmul_rn(bxy, bz[c]), thc[k]) * inv;
                         if (k == ck) {
                             cacc += w;
                         } else {
@@ -1238,16 +1257,13 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
             // row's four nodes are summed again, from the previous row's end value.
             const u32x4 rr = philox_draw(a.seed, i, sweep, 1u, chain);
             const float t = u01_f24(rr.x) * S;
-            int row = R - 1;
-            float cdf = 0.0f;
-            for (int r = 0; r < R; ++r) {
-                const float e = cps[r * kEThreads];
-                if (e >= t) {
-                    row = r;
-                    break;
-                }
-                cdf = e;
-            }
+            // (a binary search of the checkpoints: four or two dependent loads, where a scan stops
+            // a warp at its last lane's row)
+            int row = 0;
+#pragma unroll
+            for (int h = R / 2; h > 0; h >>= 1)
+                if (cps[(row + h - 1) * kEThreads] < t) row += h;
+            float cdf = row > 0 ? cps[(row - 1) * kEThreads] : 0.0f;
             const int p = row / Q, q = row % Q;
             const float bxp = p == 0 ? bx[0] : (p == 1 ? bx[1] : (p == 2 ? bx[2] : bx[3]));
             const float byq = q == 0 ? by[0] : (q == 1 ? by[1] : (q == 2 ? by[2] : by[3]));
@@ -1258,14 +1274,22 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
                 const float lyq = q == 0 ? ly[0] : (q == 1 ? ly[1] : (q == 2 ? ly[2] : ly[3]));
                 lxy = __fadd_rn(lxp, lyq);
             }
-            const uint32_t word = gather_word<DIM>(a, a.vpad, ix, iy, iz, p, q);
+            // the row's bins, picked from the registers by its index bits
+            uint32_t pick16[R];
+#pragma unroll
+            for (int e = 0; e < R; ++e) pick16[e] = pk[e];
+#pragma unroll
+            for (int h = R / 2; h > 0; h >>= 1)
+#pragma unroll
+                for (int e = 0; e < h; ++e) pick16[e] = (row & h) ? pick16[e + h] : pick16[e];
+            const uint32_t word = pick16[0];
             int pick = -1, kp = 0;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int k = (word >> (8 * c)) & 0xff;
                 const float w =
-                    LOGT ? exp2f(__fadd_rn(__fadd_rn(__fadd_rn(lxy, lz[c]), thc[k * L]), -lm))
-                         : __fmul_rn(__fmul_rn(bxy, bz[c]), thc[k * L]);
+                    LOGT ? exp2f(__fadd_rn(__fadd_rn(__fadd_rn(lxy, lz[c]), thc[k]), -lm))
+                         : __fmul_rn(__fmul_rn(bxy, bz[c]), thc[k]);
                 cdf = __fadd_rn(cdf, w);
                 if (pick < 0 && cdf >= t) {
                     pick = row * 4 + c;
@@ -1274,9 +1298,9 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
             }
             if (pick < 0) {  // unreachable (cdf ends at S >= t); keep the last neighbour
                 pick = 4 * R - 1;
-                kp = (gather_word<DIM>(a, a.vpad, ix, iy, iz, 3, Q - 1) >> 24) & 0xff;
+                kp = (pk[R - 1] >> 24) & 0xff;
             }
-            atomicAdd(&hc[kp * L + a.u[i]], 1u);
+            atomicAdd(&hc[kp * L + ui], 1u);
             const int ox = pick / (4 * Q) - 1, oy = (pick / 4) % Q - 1, oz = pick % 4 - 1;
             vp.store_r(a, i, V, fx + (float)ox, fy + (float)oy, fz + (float)oz, cs);
         }
@@ -1517,10 +1541,23 @@ int fast_threads(long V, int K, int L, bool logt, bool half) {
     return kWideThreads;
 }
 
+// row pitch of the general kernel's transposed theta: 9 banks apart from row to row where that
+// leaves room for the CTAs an SM would hold without it (lanes of one voxel bin then read different
+// banks for different node bins), else packed
+int general_pitch(int K, int L, bool sample) {
+    const size_t rest = ((size_t)K * L + (sample ? 16 * kEThreads : 0)) * sizeof(float) + 2048;
+    const size_t packed = rest + (size_t)L * K * 4, padded = rest + (size_t)L * theta_pitch(K) * 4;
+    const size_t sm = 228 * 1024;
+    const size_t most = sample ? 3 : 2;
+    const size_t want = std::min(most, sm / packed);
+    return padded * (want < 1 ? 1 : want) <= sm && padded <= 227 * 1024 ? theta_pitch(K) : K;
+}
+
 size_t estep_smem(bool sample, int K, int L, bool logt = false, bool half = false,
                   int tpb = kFastThreads) {
     if (!sample && K <= kSmallK) return fast_smem(K, L, tpb, logt, half);
-    return (size_t)(2 * K * L + (sample ? 16 * kEThreads : 0)) * sizeof(float);
+    return ((size_t)K * L + (size_t)L * general_pitch(K, L, sample) +
+            (sample ? 16 * kEThreads : 0)) * sizeof(float);
 }
 }  // namespace
 
@@ -1727,6 +1764,7 @@ void launch_estep(const EStepArgs &args, bool sample, int grid, cudaStream_t s, 
     const int ftpb = (sample || a.filter || a.ssdf)
                          ? kFastThreads
                          : fast_threads(a.V, a.K, a.L, a.logt != 0, a.halfcol != 0);
+    a.tpitch = general_pitch(a.K, a.L, sample);
     const size_t smem = a.ssdf     ? ssdf_smem(a.M, a.Fn, sample)
                         : a.filter ? filter_smem(a.K, a.L, a.M, sample)
                                    : estep_smem(sample, a.K, a.L, a.logt != 0, a.halfcol != 0,
