@@ -1,6 +1,7 @@
 // Registration / sampling engines: device buffers, CUDA-graph-captured iteration chunks and the
 // device-side convergence test of the EM loop (BINDER/src/cpu/Registration.cpp:122-217,
 // :515-642; BINDER/src/gpu/Registration.cu:839-1026).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -41,6 +42,21 @@ double spline_sigma2(int order) {
     if (order == 2) return 8.0 / (9.0 * pi);
     if (order == 1) return 0.4 * 0.4;
     return 9.0 / (8.0 * pi);
+}
+
+// `p` (freed first) becomes n slots of `slot` floats, fewer where the memory for them is not there,
+// one at least; returns their number.  The ring lives for one sampler call.
+int alloc_ring(float *&p, long slot, int n, cudaStream_t s) {
+    dfree(p, s);
+    for (;; n /= 2) {
+        try {
+            p = dalloc<float>((size_t)slot * n, s);
+            return n;
+        } catch (const Error &) {
+            if (n <= 1) throw;
+            cudaGetLastError();
+        }
+    }
 }
 
 struct Graph {
@@ -171,6 +187,11 @@ int default_precision() {
     return kPrecBF16x3;
 }
 
+bool MStep::paired() const {
+    const bool bf16 = precision == kPrecBF16x3 || precision == kPrecBF16;
+    return bf16 && !fused2d && pair_supported(nx, ny, nz, precision == kPrecBF16 ? 1 : 2);
+}
+
 void MStep::prepare_sampling(cudaStream_t s) {
     if (!noise) noise = dalloc<float>((size_t)V * 3 * chains, s);
 }
@@ -193,8 +214,10 @@ void MStep::release(cudaStream_t s) {
 void MStep::enqueue(const float *r, float *d, const float *xpos, const float *D, DevState *st,
                     double sigma2, int sample, int want_raw, int every, uint64_t seed,
                     uint32_t chain, double rho_p, const double eta2[3], const int *skip,
-                    cudaStream_t s) {
+                    cudaStream_t s, int ring_n, long ring_stride) {
     AxisArgs<float> a{};
+    a.ring_n = ring_n;
+    a.ring_stride = ring_stride;
     a.comp_stride = V;
     a.st = st;
     a.skip = skip;
@@ -225,8 +248,10 @@ void MStep::enqueue(const float *r, float *d, const float *xpos, const float *D,
                            s);
         a.noise = noise;
     }
+    BINDER_CHECK(ring_n <= 1 || (paired() && nz > 1),
+                 "a ring of positions needs the paired passes");
     // BF16 operands and axes of at most 256: two passes per launch, all components in one launch
-    if (bf16 && pair_supported(nx, ny, nz, planes)) {
+    if (paired()) {
         a.chain_comps = chains > 1 ? ncomp : 0;
         run_pairs(a, ncomp * chains, planes, s, r, d, xpos);
         return;
@@ -401,7 +426,7 @@ Registration::~Registration() {
     em_graph_.clear();
     const cudaStream_t s = own_stream_;
     dfree(d_, s); dfree(x_, s); dfree(r_, s); dfree(D_, s); dfree(theta_, s); dfree(hist_, s);
-    dfree(hcnt_, s); dfree(u_, s); dfree(vpad_, s); dfree(mean_, s);
+    dfree(hcnt_, s); dfree(u_, s); dfree(vpad_, s); dfree(mean_, s); dfree(ring_, s);
     dfree(m2_, s); dfree(hfix_, s); dfree(mpart_, s);
     dfree(stats_, s); dfree(st_, s); dfree(d0_, s); dfree(theta0_, s);
     dfree(ssd_, s); dfree(ssd0_, s); dfree(colmax_, s); dfree(colmax0_, s);
@@ -858,6 +883,19 @@ int Registration::em(int max_iterations, double convergence_th, int update, int 
     return h.iter;
 }
 
+// Slots of the sampler's ring of positions: the moments then take that many sweeps at a time.  Where
+// the paired passes write the positions and the E-step that reads them knows the ring, as many as
+// fit 3 GB, at most 8 (12 + 144 / 8 B per voxel and sweep instead of 156; more would save little).
+int Registration::sampler_ring(const MStep &m, int chains, int total, int sample_posteriors,
+                               int sample_transformation_parameters) const {
+    if (!sample_transformation_parameters || !m.paired() || N_ != 3) return 1;
+    if (sample_posteriors && lk_ != 0 && lk_ != 1) return 1;
+    const size_t slot = sizeof(float) * (size_t)V_ * N_ * chains;
+    const long fit = (long)((3ull << 30) / slot);
+    const long n = std::min({(long)kMaxRing, (long)total, fit});
+    return n < 2 ? 1 : (int)n;
+}
+
 void Registration::sampler(uint64_t seed, int N_b, int N_s, int sample_gamma,
                            int sample_gamma_every, int sample_posteriors,
                            int sample_likelihood_parameters, int sample_transformation_parameters,
@@ -885,10 +923,18 @@ void Registration::sampler(uint64_t seed, int N_b, int N_s, int sample_gamma,
     BINDER_CUDA(cudaMemsetAsync(m2_, 0, sizeof(double) * V_ * NM2, stream_));
     reset_state(true);
     const int total = N_b + N_s;
+    const long slot = (long)V_ * N_;
+    int R = sampler_ring(mstep_, 1, total, sample_posteriors, sample_transformation_parameters);
     if (total > 0 && sample_transformation_parameters) {
         mstep_.prepare_sampling(own_stream_);
+        if (R > 1) R = alloc_ring(ring_, slot, R, own_stream_);
         BINDER_CUDA(cudaStreamSynchronize(own_stream_));
     }
+    // sweep 0 reads the last slot
+    float *const pos = R > 1 ? ring_ : d_;
+    if (R > 1)
+        BINDER_CUDA(cudaMemcpyAsync(ring_ + slot * (R - 1), d_, sizeof(float) * slot,
+                                    cudaMemcpyDeviceToDevice, stream_));
     if (total > 0) {
         const double eta2[3] = {eta_[0] * eta_[0], eta_[1] * eta_[1], eta_[2] * eta_[2]};
         const double rho_p = rho_[0] * rho_[1] * rho_[2];
@@ -899,7 +945,11 @@ void Registration::sampler(uint64_t seed, int N_b, int N_s, int sample_gamma,
         const long long kernels = capture_graph(stream_, graph, [&] {
             for (int c = 0; c < chunk; ++c) {
                 if (sample_posteriors) {
-                    launch_estep(estep_args(&st_->done), true, egrid_s_, stream_);
+                    EStepArgs e = estep_args(&st_->done);
+                    e.d = pos;
+                    e.ring_n = R;
+                    e.ring_stride = slot;
+                    launch_estep(e, true, egrid_s_, stream_);
                 }
                 if (sample_likelihood_parameters) {
                     if (lk_ == 1)  // SSDLikelihood::sample_parameters from the sweep's counts
@@ -912,13 +962,13 @@ void Registration::sampler(uint64_t seed, int N_b, int N_s, int sample_gamma,
                                                 st_, stream_);
                 }
                 if (sample_transformation_parameters) {
-                    mstep_.enqueue(r_, d_, x_, D_, st_, sigma2_, 1, sample_gamma, every, seed_,
-                                   chain_, rho_p, eta2, &st_->done, stream_);
+                    mstep_.enqueue(r_, pos, x_, D_, st_, sigma2_, 1, sample_gamma, every, seed_,
+                                   chain_, rho_p, eta2, &st_->done, stream_, R, slot);
                     if (sample_gamma)
                         launch_nu_sample(st_, sample_gamma, every, N_, V_, rho_p, eta2, seed_,
                                          chain_, stream_);
                 }
-                launch_sweep_end(d_, mean_, m2_, V_, N_, N_b, total, st_, stream_);
+                launch_sweep_end(pos, mean_, m2_, V_, N_, N_b, total, st_, stream_, 1, R, slot);
             }
         });
         cudaEvent_t t0, t1;
@@ -926,6 +976,9 @@ void Registration::sampler(uint64_t seed, int N_b, int N_s, int sample_gamma,
         BINDER_CUDA(cudaEventCreate(&t1));
         BINDER_CUDA(cudaEventRecord(t0, stream_));
         for (int done = 0; done < total; done += chunk) replay(graph, kernels, stream_);
+        if (R > 1)
+            BINDER_CUDA(cudaMemcpyAsync(d_, ring_ + slot * ((total - 1) % R), sizeof(float) * slot,
+                                        cudaMemcpyDeviceToDevice, stream_));
         BINDER_CUDA(cudaEventRecord(t1, stream_));
         BINDER_CUDA(cudaEventSynchronize(t1));
         float ms = 0.0f;
@@ -948,14 +1001,15 @@ void Registration::sampler(uint64_t seed, int N_b, int N_s, int sample_gamma,
     dfree(mean_aos, stream_);
     dfree(cov_aos, stream_);
     BINDER_CUDA(cudaStreamSynchronize(stream_));
+    dfree(ring_, own_stream_);
     for (int n = 0; n < 3; ++n) gamma0_[n] = h.gamma[n];  // the prior keeps sampled gammas
 }
 
 void Registration::release_chains() {
     if (!cb_) return;
     const cudaStream_t s = own_stream_;
-    dfree(cb_->d, s); dfree(cb_->r, s); dfree(cb_->theta, s); dfree(cb_->hcnt, s);
-    dfree(cb_->st, s); dfree(cb_->mean, s); dfree(cb_->m2, s);
+    dfree(cb_->r, s); dfree(cb_->theta, s); dfree(cb_->hcnt, s);
+    dfree(cb_->st, s); dfree(cb_->mean, s); dfree(cb_->m2, s); dfree(cb_->ring, s);
     cb_->mstep.release(s);
     delete cb_;
     cb_ = nullptr;
@@ -989,7 +1043,6 @@ void Registration::sampler_chains(uint64_t seed, int chains, int N_b, int N_s, i
         release_chains();
         cb_ = new ChainBatch();
         cb_->chains = C;
-        cb_->d = dalloc<float>(VN * C, so);
         cb_->r = dalloc<float>(VN * C, so);
         cb_->theta = dalloc<float>(KL * C, so);
         cb_->hcnt = dalloc<unsigned>(KL * C, so);
@@ -1004,10 +1057,17 @@ void Registration::sampler_chains(uint64_t seed, int chains, int N_b, int N_s, i
         cb_->mstep.prepare_sampling(own_stream_);
         BINDER_CUDA(cudaStreamSynchronize(own_stream_));
     }
+    const int total = N_b + N_s;
+    const long slot = (long)(VN * C);
+    const int R = alloc_ring(cb_->ring, slot,
+                             sampler_ring(cb_->mstep, C, total, sample_posteriors,
+                                          sample_transformation_parameters), so);
+    BINDER_CUDA(cudaStreamSynchronize(so));
     ChainBatch &b = *cb_;
+    float *const start = b.ring + slot * (R - 1);  // sweep 0 reads the last slot
     // every chain starts from the object's positions, dream locations, theta and gammas
     for (int c = 0; c < C; ++c) {
-        BINDER_CUDA(cudaMemcpyAsync(b.d + VN * c, d_, sizeof(float) * VN,
+        BINDER_CUDA(cudaMemcpyAsync(start + VN * c, d_, sizeof(float) * VN,
                                     cudaMemcpyDeviceToDevice, stream_));
         BINDER_CUDA(cudaMemcpyAsync(b.r + VN * c, r_, sizeof(float) * VN,
                                     cudaMemcpyDeviceToDevice, stream_));
@@ -1029,14 +1089,13 @@ void Registration::sampler_chains(uint64_t seed, int chains, int N_b, int N_s, i
                                     cudaMemcpyHostToDevice, stream_));
         BINDER_CUDA(cudaStreamSynchronize(stream_));  // `hs` goes out of scope
     }
-    const int total = N_b + N_s;
     if (total > 0) {
         const double eta2[3] = {eta_[0] * eta_[0], eta_[1] * eta_[1], eta_[2] * eta_[2]};
         const double rho_p = rho_[0] * rho_[1] * rho_[2];
         const int every = sample_gamma_every < 1 ? 1 : sample_gamma_every;
         const int chunk = 1;  // one sweep of every chain per graph, replayed `total` times
         EStepArgs e = estep_args(&b.st->done);
-        e.d = b.d; e.r = b.r; e.theta = b.theta; e.hcnt = b.hcnt; e.st = b.st; e.seed = seed;
+        e.d = b.ring; e.ring_n = R; e.ring_stride = slot; e.r = b.r; e.theta = b.theta; e.hcnt = b.hcnt; e.st = b.st; e.seed = seed;
         Graph graph;
         const long long kernels = capture_graph(stream_, graph, [&] {
             for (int c = 0; c < chunk; ++c) {
@@ -1045,13 +1104,14 @@ void Registration::sampler_chains(uint64_t seed, int chains, int N_b, int N_s, i
                     launch_dirichlet_sample(b.theta, b.hcnt, K_, L_, alpha_, seed, chain_, b.st,
                                             stream_, C);
                 if (sample_transformation_parameters) {
-                    b.mstep.enqueue(b.r, b.d, x_, D_, b.st, sigma2_, 1, sample_gamma, every, seed,
-                                    chain_, rho_p, eta2, &b.st->done, stream_);
+                    b.mstep.enqueue(b.r, b.ring, x_, D_, b.st, sigma2_, 1, sample_gamma, every,
+                                    seed, chain_, rho_p, eta2, &b.st->done, stream_, R, slot);
                     if (sample_gamma)
                         launch_nu_sample(b.st, sample_gamma, every, N_, V_, rho_p, eta2, seed,
                                          chain_, stream_, C);
                 }
-                launch_sweep_end(b.d, b.mean, b.m2, V_, N_, N_b, total, b.st, stream_, C);
+                launch_sweep_end(b.ring, b.mean, b.m2, V_, N_, N_b, total, b.st, stream_, C, R,
+                                 slot);
             }
         });
         cudaEvent_t t0, t1;
@@ -1103,6 +1163,7 @@ void Registration::sampler_chains(uint64_t seed, int chains, int N_b, int N_s, i
     dfree(mstage, stream_);
     dfree(cstage, stream_);
     BINDER_CUDA(cudaStreamSynchronize(stream_));
+    dfree(b.ring, so);
 }
 
 double Registration::profile_stage(int stage, int n) {

@@ -50,7 +50,10 @@ struct MStep {
     void release(cudaStream_t s);
     void enqueue(const float *r, float *d, const float *xpos, const float *D, DevState *st,
                  double sigma2, int sample, int want_raw, int every, uint64_t seed, uint32_t chain,
-                 double rho_p, const double eta2[3], const int *skip, cudaStream_t s);
+                 double rho_p, const double eta2[3], const int *skip, cudaStream_t s,
+                 int ring_n = 1, long ring_stride = 0);
+    // whether enqueue() runs the paired passes, whose last one can write a ring of positions
+    bool paired() const;
     void run_chain(AxisArgs<float> a, int c0, int nc, cudaStream_t s, const float *r, float *d,
                    const float *xpos, bool tc, int planes);
     void run_pairs(AxisArgs<float> a, int nc, int planes, cudaStream_t s, const float *r, float *d,
@@ -203,6 +206,7 @@ class Registration {
     unsigned long long *hfix_ = nullptr;  // order-independent EM histogram merge (EStepArgs)
     double *mpart_ = nullptr;
     double *mean_ = nullptr, *m2_ = nullptr, *stats_ = nullptr;
+    float *ring_ = nullptr;  // positions of the last sweeps, during a sampler call (sampler_ring)
     int stats_cap_ = 0;
     DevState *st_ = nullptr;
     MStep mstep_;
@@ -210,14 +214,17 @@ class Registration {
     // buffers of the last batch of chains (kept for the next call with the same count)
     struct ChainBatch {
         int chains = 0;
-        float *d = nullptr, *r = nullptr, *theta = nullptr;
+        float *r = nullptr, *theta = nullptr;
         unsigned *hcnt = nullptr;
         DevState *st = nullptr;
         double *mean = nullptr, *m2 = nullptr;
+        float *ring = nullptr;  // positions of the last sweeps, during a call (sampler_ring)
         MStep mstep;
     };
     ChainBatch *cb_ = nullptr;
     void release_chains();
+    int sampler_ring(const MStep &m, int chains, int total, int sample_posteriors,
+                     int sample_transformation_parameters) const;
     int estep_grid_override_ = 0;
     // likelihood / prior parameters
     bool have_mi_ = false, have_tr_ = false;

@@ -1133,13 +1133,17 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
     __syncthreads();
 
     const uint32_t sweep = SAMPLE ? (uint32_t)st->sweep : 0u;
+    // the slot of the positions the last sweep left
+    const long rs = SAMPLE && a.ring_n > 1
+                        ? cs + (long)((sweep + a.ring_n - 1) % a.ring_n) * a.ring_stride
+                        : cs;
     double mll = 0.0;
     unsigned long long deg = 0;
     const unsigned V = (unsigned)a.V, nz = (unsigned)a.nz, ny = (unsigned)a.ny;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x) {
         VoxelPos<DIM> vp;
         // positions far outside any grid (or non-finite) are degenerate: keep them as they are
-        if (!vp.load(a, i, V, ny, nz, cs)) {
+        if (!vp.load(a, i, V, ny, nz, rs)) {
             vp.store_r(a, i, V, vp.px, vp.py, vp.pz, cs);
             ++deg;
             continue;
@@ -1469,10 +1473,15 @@ __global__ void em_finish_kernel(DevState *st, double *stats, int max_iter, doub
 
 // Registration.cpp:593-623 in FP64 with the symmetric M2 (xx, xy, xz, yy, yz, zz)
 // N components: mean [N][V], M2 as its upper triangle [N (N + 1) / 2][V] (row-major: xx, xy, xz,
-// yy, yz, zz or xx, xy, yy)
+// yy, yz, zz or xx, xy, yy).
+// HBM-bound: a sweep's update alone reads and writes every moment (156 B per voxel at N = 3; 0.95 ms
+// per sweep of 32 chains at 96^3, 4.7 TB/s).  With ring_n sweeps' positions kept, one launch applies
+// their updates one after another in registers -- the same operations in the same order -- and the
+// moments move once per ring_n sweeps: 12 + 144 / ring_n B per voxel and sweep.
 template <int N>
-__global__ void sweep_end_kernel(const float *d, double *mean, double *m2, long V, int N_b,
-                                 DevState *st) {
+__global__ void __launch_bounds__(256) sweep_end_kernel(const float *d, double *mean, double *m2,
+                                                        long V, int N_b, int total, int ring_n,
+                                                        long ring_stride, DevState *st) {
     // chain blockIdx.y of a batch: positions [N][V], mean [N][V], M2 [N (N + 1) / 2][V] per chain
     d += (long)blockIdx.y * N * V;
     mean += (long)blockIdx.y * N * V;
@@ -1480,26 +1489,45 @@ __global__ void sweep_end_kernel(const float *d, double *mean, double *m2, long 
     st += blockIdx.y;
     if (st->done) return;
     const int sweep = st->sweep;
-    if (sweep >= N_b) {
-        const double inv_n = 1.0 / ((double)(sweep - N_b) + 1.0);
-        for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < V;
-             i += (long)gridDim.x * blockDim.x) {
+    const int slot = sweep % ring_n;
+    if (sweep < N_b || (slot != ring_n - 1 && sweep + 1 < total)) return;
+    // sweeps first .. sweep, in slots sweep's slot - n + 1 .. its slot (a flush empties the ring)
+    const int first = sweep - slot > N_b ? sweep - slot : N_b;
+    const int n = sweep - first + 1;
+    __shared__ double inv_n[kMaxRing];
+    if ((int)threadIdx.x < n) inv_n[threadIdx.x] = 1.0 / ((double)(first + threadIdx.x - N_b) + 1.0);
+    __syncthreads();
+    const float *p0 = d + (long)(slot - n + 1) * ring_stride;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < V;
+         i += (long)gridDim.x * blockDim.x) {
+        constexpr int M = N * (N + 1) / 2;
+        double mo[N], acc[M];
+#pragma unroll
+        for (int c = 0; c < N; ++c) mo[c] = mean[c * V + i];
+#pragma unroll
+        for (int e = 0; e < M; ++e) acc[e] = m2[e * V + i];
+        const float *p = p0 + i;
+#pragma unroll 4
+        for (int s = 0; s < n; ++s, p += ring_stride) {
+            const double w = inv_n[s];
             double d1[N], d2[N];
 #pragma unroll
-            for (int n = 0; n < N; ++n) {
-                const double val = (double)d[n * V + i];
-                const double mo = mean[n * V + i];
-                d1[n] = val - mo;
-                const double mn = mo + d1[n] * inv_n;
-                mean[n * V + i] = mn;
-                d2[n] = val - mn;
+            for (int c = 0; c < N; ++c) {
+                const double val = (double)p[c * V];
+                d1[c] = val - mo[c];
+                mo[c] = mo[c] + d1[c] * w;
+                d2[c] = val - mo[c];
             }
             int e = 0;
 #pragma unroll
             for (int r = 0; r < N; ++r)
 #pragma unroll
-                for (int c = r; c < N; ++c, ++e) m2[e * V + i] += d1[r] * d2[c];
+                for (int c = r; c < N; ++c, ++e) acc[e] += d1[r] * d2[c];
         }
+#pragma unroll
+        for (int c = 0; c < N; ++c) mean[c * V + i] = mo[c];
+#pragma unroll
+        for (int e = 0; e < M; ++e) m2[e * V + i] = acc[e];
     }
 }
 
@@ -2046,7 +2074,9 @@ void launch_em_finish(DevState *st, double *stats, int max_iter, double th, doub
 }
 
 void launch_sweep_end(const float *d, double *mean, double *m2, long V, int N, int N_b,
-                      int total, DevState *st, cudaStream_t s, int chains) {
+                      int total, DevState *st, cudaStream_t s, int chains, int ring_n,
+                      long ring_stride) {
+    BINDER_CHECK(ring_n >= 1 && ring_n <= kMaxRing, "the position ring has 1 to 8 slots");
     int dev = 0, sms = 148;
     BINDER_CUDA(cudaGetDevice(&dev));
     BINDER_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -2055,8 +2085,12 @@ void launch_sweep_end(const float *d, double *mean, double *m2, long V, int N, i
     if (chains > 1) g = (g + chains - 1) / chains;  // the same total CTAs over the chains
     const dim3 grid((unsigned)g, (unsigned)chains);
     BINDER_CHECK(N == 2 || N == 3, "Welford moments need N = 2 or 3");
-    if (N == 3) count_launch(), sweep_end_kernel<3><<<grid, 256, 0, s>>>(d, mean, m2, V, N_b, st);
-    else count_launch(), sweep_end_kernel<2><<<grid, 256, 0, s>>>(d, mean, m2, V, N_b, st);
+    if (N == 3)
+        count_launch(), sweep_end_kernel<3><<<grid, 256, 0, s>>>(d, mean, m2, V, N_b, total, ring_n,
+                                                                 ring_stride, st);
+    else
+        count_launch(), sweep_end_kernel<2><<<grid, 256, 0, s>>>(d, mean, m2, V, N_b, total, ring_n,
+                                                                 ring_stride, st);
     BINDER_CUDA(cudaGetLastError());
     launch_sweep_advance(st, total, s, chains);
 }

@@ -11,6 +11,10 @@ struct SsdfState;
 
 struct EStepArgs {
     const float *d;   // positions, SoA [dim][V] (node-grid coordinates)
+    // the sampling E-step of the MI and SSD likelihoods with ring_n > 1: `d` has ring_n slots
+    // ring_stride elements apart and sweep s reads slot (s - 1) % ring_n
+    int ring_n;
+    long ring_stride;
     float *r;         // out: dream location minus voxel position, SoA [dim][V]
     const float *x;   // voxel positions SoA [dim][V], or null for the identity grid
     const uint8_t *u;     // fixed-image bins [V]
@@ -150,9 +154,13 @@ void launch_nu_sample(DevState *st, int sample_gamma, int every, int N, long V, 
 void launch_em_finish(DevState *st, double *stats, int max_iter, double th, double nzv,
                       cudaStream_t s);
 // Welford mean [N][V] / symmetric M2 [N (N + 1) / 2][V] update in FP64 when sweep >= N_b, then
-// sweep += 1 (done once sweep reaches `total`)
+// sweep += 1 (done once sweep reaches `total`).  With ring_n > 1 the positions of sweep s are in
+// slot s % ring_n of d (ring_stride elements apart) and the moments take ring_n sweeps at a time,
+// in their order, with the last slot and with the last sweep.
+constexpr int kMaxRing = 8;
 void launch_sweep_end(const float *d, double *mean, double *m2, long V, int N, int N_b,
-                      int total, DevState *st, cudaStream_t s, int chains = 1);
+                      int total, DevState *st, cudaStream_t s, int chains = 1, int ring_n = 1,
+                      long ring_stride = 0);
 // sweep += 1 (done once sweep reaches `total`)
 void launch_sweep_advance(DevState *st, int total, cudaStream_t s, int chains = 1);
 

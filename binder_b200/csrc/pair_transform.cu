@@ -79,6 +79,8 @@ struct PairArgs {
     const float *xpos;
     int dims;
     int comp0, chain_comps;
+    int ring_n;
+    long ring_stride;
     const int *skip;
 };
 
@@ -477,6 +479,9 @@ __global__ void __launch_bounds__((NL + NE + 2) * 32, NE == 4 ? 2 : 1) pair_kern
                 for (int m = 0; m < 16; ++m, at += ks) v[m] = m < left ? __ldg(p + at) : 0.0f;
             }
         };
+        const long ring = KIND == kPairInverse && a.ring_n > 1
+                              ? (long)(a.st->sweep % a.ring_n) * a.ring_stride
+                              : 0;
         Tile t = tile_at<KIND>(a, 0);
         if (KIND == kPairSpectral)
             load_col(a.D + t.row0, 2 * part, (long)t.row0 + row < a.lines, dnext);
@@ -575,7 +580,7 @@ __global__ void __launch_bounds__((NL + NE + 2) * 32, NE == 4 ? 2 : 1) pair_kern
             ok = !__any_sync(0xffffffffu, !ok || *err);
             if (!ok) break;
             umma::fence_after_sync();
-            float *o = a.out + t.base;
+            float *o = a.out + t.base + ring;
             if (KIND == kPairInverse) {
                 for (int mt = 0; mt * 128 < a.np2; ++mt) {
                     const int z = mt * 128 + (int)row;
@@ -804,7 +809,7 @@ void launch_pair_pass(const AxisArgs<float> &b, PairKind kind, int nx, int ny, i
     a.every = b.every < 1 ? 1 : b.every; a.noise = b.noise; a.rho_p = b.rho_p;
     for (int i = 0; i < 3; ++i) a.eta2[i] = b.eta2[i];
     a.xpos = b.xpos; a.dims = b.dims; a.comp0 = b.comp0; a.chain_comps = b.chain_comps;
-    a.skip = b.skip;
+    a.ring_n = b.ring_n; a.ring_stride = b.ring_stride; a.skip = b.skip;
     if (planes == 2) launch_planes<2>(kind, a, p, s);
     else launch_planes<1>(kind, a, p, s);
 }

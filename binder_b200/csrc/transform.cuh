@@ -73,6 +73,10 @@ struct AxisArgs {
     // a batch of chains: components chain * chain_comps + n (n < chain_comps) with states
     // st[chain] and Philox chain indices chain + chain; 0 for one chain
     int chain_comps;
+    // kPairInverse with ring_n > 1: the positions go to slot st->sweep % ring_n of `out`, the slots
+    // ring_stride elements apart
+    int ring_n;
+    long ring_stride;
 };
 
 // The prior-sampling normals of every coefficient: noise[c * V + i] = dct_prior_normal(seed, i,
