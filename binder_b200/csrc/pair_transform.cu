@@ -164,8 +164,8 @@ __device__ __forceinline__ Tile tile_at(const PairArgs &a, int i) {
 template <int KIND, int PLANES, int NL, int NE, bool VAR>
 __global__ void __launch_bounds__((NL + NE + 2) * 32, NE == 4 ? 2 : 1) pair_kernel(const PairArgs a) {
     constexpr int kMma = NL + NE;  // the MMA warp
-    // the load warps work in groups on alternate steps, so two steps are in flight
-    constexpr int kGroups = KIND == kPairSpectral ? 1 : 2;
+    // eight load warps or more work in two groups on alternate steps: two steps in flight
+    constexpr int kGroups = NL >= 8 ? 2 : 1;
     constexpr int GW = NL / kGroups;  // warps per group
     if (a.skip && *a.skip) return;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -671,7 +671,8 @@ struct PairShape {
     long ctas;  // tiles per component
 };
 
-PairShape pair_shape(PairKind kind, int nx, int ny, int nz, int planes, int ncomp) {
+PairShape pair_shape(PairKind kind, int nx, int ny, int nz, int planes, int ncomp,
+                     bool sample) {
     PairShape p{};
     if (nx > kMaxAxis || ny > kMaxAxis || nz > kMaxAxis) return p;
     const uint32_t pb = (uint32_t)planes * 32u;
@@ -708,14 +709,23 @@ PairShape pair_shape(PairKind kind, int nx, int ny, int nz, int planes, int ncom
     auto total = [&](int ring, int mats) {
         return fixed + (size_t)ring * xslot + (size_t)mats * p.mat_slot;
     };
-    // two CTAs of 4 + 4 warps per SM where their tables and accumulators fit and there are tiles
-    // for them, else one CTA of 8 + 8 (4 + 12 for the prior scaling, whose epilogue has most to do)
-    // (a group of four load warps covers 128 rows in its four tasks)
-    const bool two = kind != kPairSpectral && p.rp <= 128 && p.ncols <= 256 &&
-                     total(2, 2) <= 112 * 1024 && p.ctas * ncomp > 148;
+    // Two CTAs per SM where their tables and accumulators fit and there are tiles for them (a group
+    // of four load warps covers 128 rows in its four tasks), else one.  Load + epilogue warps:
+    //   forward, inverse  8 + 4 of two CTAs, 16 + 8 of one;
+    //   spectral          4 + 4 of two CTAs (14.7 us at 91x109x91; 4 + 12 of one 19.3, 8 + 4 of two
+    //                     16.9, which spill), 8 + 12 of one (55 us at 160x192x160; 4 + 12 58);
+    //   with the noise    4 + 12 of one (424 us per sweep of 32 chains at 96^3; 8 + 12 503 and
+    //                     8 + 8 526, with spills; 4 + 4 of two the same 423).
+    const bool two = !sample && p.rp <= 128 && p.ncols <= 256 && total(2, 2) <= 112 * 1024 &&
+                     p.ctas * ncomp > 148;
     const size_t limit = two ? 112 * 1024 : 226 * 1024;
-    p.nl = kind == kPairSpectral ? 4 : (two ? 8 : 16);
-    p.ne = two ? 4 : (kind == kPairSpectral ? 12 : 8);
+    if (kind == kPairSpectral) {
+        p.nl = two || sample ? 4 : 8;
+        p.ne = two ? 4 : 12;
+    } else {
+        p.nl = two ? 8 : 16;
+        p.ne = two ? 4 : 8;
+    }
     p.ring = 2;
     p.mats = 2;
     if (total(p.ring, 2) > limit) return p;
@@ -754,7 +764,12 @@ void launch(const PairArgs &a, const PairShape &p, cudaStream_t s) {
 template <int KIND, int PLANES, bool VAR>
 void launch_kind(const PairArgs &a, const PairShape &p, cudaStream_t s) {
     if constexpr (KIND == kPairSpectral) {
-        launch<KIND, PLANES, 4, 12, VAR>(a, p, s);
+        if constexpr (VAR) {
+            launch<KIND, PLANES, 4, 12, VAR>(a, p, s);
+        } else {
+            if (p.ne == 12) launch<KIND, PLANES, 8, 12, VAR>(a, p, s);
+            else launch<KIND, PLANES, 4, 4, VAR>(a, p, s);
+        }
     } else {
         if (p.ne == 8) launch<KIND, PLANES, 16, 8, VAR>(a, p, s);
         else launch<KIND, PLANES, 8, 4, VAR>(a, p, s);
@@ -779,9 +794,10 @@ void launch_planes(PairKind kind, const PairArgs &a, const PairShape &p, cudaStr
 }  // namespace
 
 bool pair_supported(int nx, int ny, int nz, int planes) {
-    if (nz == 1) return pair_shape(kPairSpectral, nx, ny, nz, planes, 1).smem > 0;
+    // (the one-CTA forms, which the two-CTA forms are smaller than)
+    if (nz == 1) return pair_shape(kPairSpectral, nx, ny, nz, planes, 1, false).smem > 0;
     for (PairKind k : {kPairForward, kPairSpectral, kPairInverse})
-        if (pair_shape(k, nx, ny, nz, planes, 1).smem == 0) return false;
+        if (pair_shape(k, nx, ny, nz, planes, 1, false).smem == 0) return false;
     return true;
 }
 
@@ -789,7 +805,7 @@ void launch_pair_pass(const AxisArgs<float> &b, PairKind kind, int nx, int ny, i
                       const UmmaMatrix &M1, const UmmaMatrix &M2, int ncomp, int planes,
                       cudaStream_t s) {
     BINDER_CHECK(planes == 1 || planes == 2, "planes must be 1 (one product) or 2 (split)");
-    const PairShape p = pair_shape(kind, nx, ny, nz, planes, ncomp);
+    const PairShape p = pair_shape(kind, nx, ny, nz, planes, ncomp, kind == kPairSpectral && b.sample);
     BINDER_CHECK(p.smem > 0, "the volume does not fit the paired transform passes");
     const int n1 = kind == kPairForward ? nz : (kind == kPairSpectral ? nx : ny);
     const int n2 = kind == kPairForward ? ny : (kind == kPairSpectral ? nx : nz);
