@@ -1,0 +1,260 @@
+// FP64 Hartley transforms H[k] = sum_j x[j] cas(2 pi j k / n) along one axis, on the FP64 matrix
+// instructions.
+//
+// Folding: with e_j = x_j + x_{n-j} and o_j = x_j - x_{n-j} (j = 1 .. n/2; x_0, and x_{n/2} of an
+// even n, in e alone), C_k = sum_j e_j cos(2 pi j k / n) and S_k = sum_j o_j sin(2 pi j k / n) for
+// k = 0 .. n/2 give H[k] = C_k + S_k and H[n-k] = C_k - S_k: two products of (n/2)^2 instead of one
+// of n^2, half the operations.
+//
+// A CTA of four warps owns 32 lines.  It folds them into shared memory (e and o, [j][32] with a
+// pitch of 36 doubles: the four rows of a fragment are 8 banks apart), and warp w computes the
+// 8-row tiles w, w + 4, ... of both products for all 32 lines with mma.m8n8k4 (FP64 in, FP64 FMA
+// accumulation), the matrices coming from global memory through L1.  kHartleyPoisson folds the
+// scaled coefficients straight from the accumulators -- a thread holds k and n - k of its lines --
+// and transforms again, so the spectrum is never stored.
+//
+// Bound: the FP64 pipe (0.5 n FMA per element and pass; 5.1 GFLOP per pass at 160x192x160, 0.14 ms at
+// 36 TFLOP/s).  Three components at 160x192x160, z / y / x with the Poisson scaling: 0.21 / 0.29 /
+// 0.34 ms, where a 64-line register-blocked FMA kernel of the unfolded matrix took 0.6 / 0.95 / 0.95
+// (one CTA of eight warps per SM, its staging not overlapped, a division per staged element).
+// 32 lines and four warps per CTA, so that two or three CTAs share an SM and one's folding overlaps
+// another's products.
+#include <cmath>
+#include <vector>
+
+#include "hartley.cuh"
+#include "layout.cuh"
+
+namespace binder {
+namespace {
+
+constexpr int kLinesH = 32;  // lines per CTA
+constexpr int kPitchH = 36;  // doubles per row of e / o
+constexpr int kThreadsH = 128;
+
+struct HArgs {
+    HartleyArgs a;
+    const double *cs, *sn;
+    int n, cols, tiles;  // tiles: 8-row tiles of the halves
+    long nlines;
+};
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+
+// both products of this warp's tiles: cC = cos e, cS = sin o
+template <int U>
+__device__ __forceinline__ void products(const HArgs &h, const double *E, const double *O,
+                                         double (&cC)[U][4][2], double (&cS)[U][4][2], int warp,
+                                         int lane) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) cC[u][t][0] = cC[u][t][1] = cS[u][t][0] = cS[u][t][1] = 0.0;
+    const int ar = lane >> 2, ak = lane & 3;
+    const double *pc[U], *ps[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        // tiles past the last one repeat it: their results are not stored
+        const int m = min(warp + 4 * u, h.tiles - 1);
+        pc[u] = h.cs + (long)(m * 8 + ar) * h.cols + ak;
+        ps[u] = h.sn + (long)(m * 8 + ar) * h.cols + ak;
+    }
+    double a0[U], a1[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) a0[u] = __ldg(pc[u]), a1[u] = __ldg(ps[u]);
+    for (int j = 0; j < h.cols; j += 4) {
+        double n0[U], n1[U];  // the next step's matrix fragments, in flight during this one
+        const int jn = j + 4 < h.cols ? j + 4 : j;
+#pragma unroll
+        for (int u = 0; u < U; ++u) n0[u] = __ldg(pc[u] + jn), n1[u] = __ldg(ps[u] + jn);
+        const double *e = E + (j + ak) * kPitchH + ar, *o = O + (j + ak) * kPitchH + ar;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const double be = e[t * 8], bo = o[t * 8];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                dmma(cC[u][t], a0[u], be);
+                dmma(cS[u][t], a1[u], bo);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) a0[u] = n0[u], a1[u] = n1[u];
+    }
+}
+
+template <int U, int MODE>
+__global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(const HArgs h) {
+    extern __shared__ __align__(16) double sm[];
+    double *E = sm, *O = sm + (long)h.cols * kPitchH;
+    const HartleyArgs &a = h.a;
+    const int n = h.n, half = n >> 1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int comp = blockIdx.y;
+    const double *in = a.in + comp * a.V;
+    double *out = a.out + comp * a.V;
+    const bool contig = a.s == 1;
+    long base;  // first element of the tile
+    int nl;     // lines of the tile
+    long t0 = 0;
+    if (contig) {
+        const long l0 = (long)blockIdx.x * kLinesH;
+        nl = (int)min((long)kLinesH, a.outer - l0);
+        base = l0 * n;
+    } else {
+        const long tiles = (a.s + kLinesH - 1) / kLinesH;
+        const long o = blockIdx.x / tiles;
+        t0 = (blockIdx.x - o * tiles) * kLinesH;
+        nl = (int)min((long)kLinesH, a.s - t0);
+        base = o * n * a.s + t0;
+    }
+    const long js = contig ? 1 : a.s, ls = contig ? n : 1;  // strides of j and of the lines
+    // ---- fold: contiguous lines 8 j x 4 lines per warp instruction (64-byte segments), strided
+    // ones 32 neighbouring lines
+    const int lj = contig ? lane & 7 : 0, ll = contig ? lane >> 3 : lane;
+    for (int c0 = 0; c0 < kLinesH; c0 += contig ? 4 : kLinesH)
+        for (int j = (contig ? warp * 8 : warp) + lj; j < h.cols; j += contig ? 32 : 4) {
+            const int c = c0 + ll;
+            double e = 0.0, o = 0.0;
+            if (c < nl && j <= half) {
+                const double *p = in + base + c * ls;
+                const double x = p[j * js];
+                if (j == 0 || 2 * j == n) {
+                    e = x;
+                } else {
+                    const double y = p[(n - j) * js];
+                    e = x + y;
+                    o = x - y;
+                }
+            }
+            E[j * kPitchH + c] = e;
+            O[j * kPitchH + c] = o;
+        }
+    __syncthreads();
+    double cC[U][4][2], cS[U][4][2];
+    products<U>(h, E, O, cC, cS, warp, lane);
+    // this thread's rows k = 8 m + lane / 4 and lines t * 8 + 2 (lane % 4) + {0, 1}
+    const int kr = lane >> 2, lc = (lane & 3) * 2;
+    if (MODE == kHartleyPoisson) {
+        __syncthreads();  // every warp has read e and o
+        const double inv_total = 1.0 / ((double)n * (double)a.s);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int c = t * 8 + lc + q;
+                const long tt = min(t0 + c, a.s - 1);
+                const int ky = (int)(tt / a.nz), kz = (int)(tt - (long)ky * a.nz);
+                const double cz = __ldg(a.cos_z + kz), cy = __ldg(a.cos_y + ky);
+                auto scale = [&](double v, int k) {
+                    const double lam = 6.0 - 2.0 * cz - 2.0 * __ldg(a.cos_x + k) - 2.0 * cy;
+                    return fabs(lam) > 1e-10 ? -v / lam * inv_total : 0.0;
+                };
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int k = (warp + 4 * u) * 8 + kr;
+                    if (warp + 4 * u >= h.tiles || k > half) continue;
+                    const double C = cC[u][t][q], S = cS[u][t][q];
+                    double e = scale(C + S, k), o = 0.0;
+                    if (k != 0 && 2 * k != n) {
+                        const double y = scale(C - S, n - k);
+                        o = e - y;
+                        e = e + y;
+                    }
+                    E[k * kPitchH + c] = e;
+                    O[k * kPitchH + c] = o;
+                }
+            }
+        __syncthreads();
+        products<U>(h, E, O, cC, cS, warp, lane);
+    }
+    const double sc = MODE == kHartleyScaled ? a.out_scale[comp] : 1.0;
+    const double of = MODE == kHartleyScaled ? a.out_offset[comp] : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int k = (warp + 4 * u) * 8 + kr;
+        if (warp + 4 * u >= h.tiles || k > half) continue;
+        const bool pair = k != 0 && 2 * k != n;
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int c = t * 8 + lc + q;
+                if (c >= nl) continue;
+                double *p = out + base + c * ls;
+                double x = cC[u][t][q] + cS[u][t][q], y = cC[u][t][q] - cS[u][t][q];
+                if (MODE == kHartleyScaled) x = x * sc + of, y = y * sc + of;
+                p[k * js] = x;
+                if (pair) p[(n - k) * js] = y;
+            }
+    }
+}
+
+template <int U, int MODE>
+void launch_u(const HArgs &h, int ncomp, cudaStream_t s) {
+    const size_t smem = (size_t)2 * h.cols * kPitchH * sizeof(double);
+    BINDER_CUDA(cudaFuncSetAttribute(hartley_kernel<U, MODE>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const long gx = h.a.s == 1 ? (h.a.outer + kLinesH - 1) / kLinesH
+                               : h.a.outer * ((h.a.s + kLinesH - 1) / kLinesH);
+    BINDER_CHECK(gx < (1L << 31), "transform grid too large");
+    count_launch(), hartley_kernel<U, MODE><<<dim3((unsigned)gx, (unsigned)ncomp), kThreadsH, smem,
+                                             s>>>(h);
+    BINDER_CUDA(cudaGetLastError());
+}
+
+template <int MODE>
+void launch_mode_h(const HArgs &h, int ncomp, cudaStream_t s) {
+    switch ((h.tiles + 3) / 4) {
+        case 1: launch_u<1, MODE>(h, ncomp, s); break;
+        case 2: launch_u<2, MODE>(h, ncomp, s); break;
+        case 3: launch_u<3, MODE>(h, ncomp, s); break;
+        case 4: launch_u<4, MODE>(h, ncomp, s); break;
+        default: launch_u<5, MODE>(h, ncomp, s); break;
+    }
+}
+
+}  // namespace
+
+void HartleyMatrix::init(int n_, cudaStream_t s) {
+    n = n_;
+    rows = (n / 2 + 1 + 7) / 8 * 8;
+    cols = (n / 2 + 1 + 3) / 4 * 4;
+    std::vector<double> host((size_t)2 * rows * cols, 0.0);
+    const double pi = 3.14159265358979323846;
+    for (int k = 0; k <= n / 2; ++k)
+        for (int j = 0; j <= n / 2; ++j) {
+            const double ang = 2.0 * pi * (double)(((long)j * k) % n) / n;
+            host[(size_t)k * cols + j] = std::cos(ang);
+            host[(size_t)(rows + k) * cols + j] = std::sin(ang);
+        }
+    dev = dev_alloc_n<double>(host.size(), s);
+    BINDER_CUDA(cudaMemcpyAsync(dev, host.data(), host.size() * sizeof(double),
+                                cudaMemcpyHostToDevice, s));
+    BINDER_CUDA(cudaStreamSynchronize(s));  // `host` goes out of scope
+}
+
+void HartleyMatrix::release(cudaStream_t s) { dev_free_p(dev, s); }
+
+void launch_hartley(const HartleyArgs &a, const HartleyMatrix &H, HartleyMode mode, int ncomp,
+                    cudaStream_t s) {
+    BINDER_CHECK(H.n >= 1 && H.n <= 256, "transform axis length must be in [1, 256]");
+    BINDER_CHECK(mode != kHartleyPoisson || a.outer == 1,
+                 "the Poisson scaling runs on the outermost axis");
+    HArgs h{};
+    h.a = a;
+    h.cs = H.dev;
+    h.sn = H.dev + (size_t)H.rows * H.cols;
+    h.n = H.n;
+    h.cols = H.cols;
+    h.tiles = H.rows / 8;
+    switch (mode) {
+        case kHartleyPlain: launch_mode_h<kHartleyPlain>(h, ncomp, s); break;
+        case kHartleyScaled: launch_mode_h<kHartleyScaled>(h, ncomp, s); break;
+        case kHartleyPoisson: launch_mode_h<kHartleyPoisson>(h, ncomp, s); break;
+    }
+}
+
+}  // namespace binder

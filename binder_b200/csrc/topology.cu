@@ -9,8 +9,8 @@
 #include <vector>
 
 #include "layout.cuh"
+#include "hartley.cuh"
 #include "topology.cuh"
-#include "transform.cuh"
 
 namespace binder {
 
@@ -167,9 +167,10 @@ __global__ void jacobian2d_kernel(const double *f, long ps, long cs, int nx, int
 
 // topology_correction_3D.cpp:488-607: the 8 vertex Jacobians of every cell, in the vertex order
 // 000, 100, 010, 001, 011, 101, 110, 111, each from the three cell edges through its vertex.
-// Positions are SoA [3][V].
+// Positions are SoA [3][V].  The limiter asks only which of them lie outside [e1, e2]: bit c of
+// mask[cell] (storing the eight values moved 64 B per cell and took twice as long).
 __global__ void corner_kernel(const double *pos, int nx, int ny, int nz, double vol, double e1,
-                              double e2, double *Jc, Red *red) {
+                              double e2, uint8_t *mask, Red *red) {
     const long V = (long)nx * ny * nz;
     const long cy = ny - 1, cz = nz - 1;
     const long cells = (long)(nx - 1) * cy * cz;
@@ -179,6 +180,7 @@ __global__ void corner_kernel(const double *pos, int nx, int ny, int nz, double 
     for (long cell = (long)blockIdx.x * blockDim.x + threadIdx.x; cell < cells;
          cell += (long)gridDim.x * blockDim.x) {
         const int x = (int)(cell / (cy * cz)), y = (int)((cell / cz) % cy), z = (int)(cell % cz);
+        unsigned bits = 0;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             const int vx = vert[c][0], vy = vert[c][1], vz = vert[c][2];
@@ -198,10 +200,11 @@ __global__ void corner_kernel(const double *pos, int nx, int ny, int nz, double 
             double j = det3(col[0][0], col[1][0], col[2][0], col[0][1], col[1][1], col[2][1],
                             col[0][2], col[1][2], col[2][2]);
             j *= vol;
-            Jc[cell * 8 + c] = j;
             lb += j < e1;
             la += j > e2;
+            bits |= (j < e1 || j > e2) ? 1u << c : 0u;
         }
+        mask[cell] = (uint8_t)bits;
     }
     for (int o = 16; o > 0; o >>= 1) {
         lb += __shfl_xor_sync(0xffffffffu, lb, o);
@@ -234,21 +237,6 @@ __global__ void gradient_kernel(const double *pos, int nx, int ny, int nz, doubl
             g[(n1 * 3 + 1) * V + p] = (pos[n1 * V + py] - c) / vs[n1];
             g[(n1 * 3 + 2) * V + p] = (pos[n1 * V + pz] - c) / vs[n1];
         }
-    }
-}
-
-__global__ void flag_cells_kernel(const double *Jc, int nx, int ny, int nz, double e1, double e2,
-                                  int *list, Red *red) {
-    const long cells = (long)(nx - 1) * (ny - 1) * (nz - 1);
-    for (long cell = (long)blockIdx.x * blockDim.x + threadIdx.x; cell < cells;
-         cell += (long)gridDim.x * blockDim.x) {
-        bool any = false;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const double j = Jc[cell * 8 + c];
-            any |= (j < e1 || j > e2);
-        }
-        if (any) list[atomicAdd(&red->count, 1)] = (int)cell;
     }
 }
 
@@ -343,69 +331,282 @@ __device__ __forceinline__ void limit_corner_lanes(double (&J)[2][2], double e1,
 
 // topology_correction_3D.cpp:247-332.  The reference visits cells in lexicographic order and a
 // cell's 8 corners in order; a cell reads and writes gradients only inside its 2x2x2 footprint,
-// so two cells interact only if they differ by at most 1 along every axis.  Level 4x + 2y + z
-// orders every such pair exactly as the lexicographic walk does and never puts two of them on
-// the same level, so processing levels in increasing order (cells of one level in parallel)
-// reproduces the sequential result exactly.  One CTA of 256 threads; levels are separated by
-// __syncthreads.
-__global__ void __launch_bounds__(256) limiter_kernel(const int *list, int *sorted, const double *Jc,
-                                                       double *g, int nx, int ny, int nz,
-                                                       double e1, double e2, int nlev, Red *red,
-                                                       unsigned *flags) {
-    extern __shared__ int sh[];
-    int *off = sh;             // nlev + 1
-    int *cur = sh + nlev + 1;  // nlev
-    const long V = (long)nx * ny * nz;
-    const long cy = ny - 1, cz = nz - 1;
-    const int n = red->count;
-    for (int l = threadIdx.x; l < nlev + 1; l += blockDim.x) off[l] = 0;
-    __syncthreads();
-    for (int q = threadIdx.x; q < n; q += blockDim.x) {
-        const long cell = list[q];
-        const int x = (int)(cell / (cy * cz)), y = (int)((cell / cz) % cy), z = (int)(cell % cz);
-        atomicAdd(&off[4 * x + 2 * y + z + 1], 1);
+// so two cells interact only if they differ by at most 1 along every axis.  A flagged cell may
+// therefore go as soon as its flagged neighbours that come before it have gone: cells with none go
+// first (round 0), and each cell counts down its later neighbours, the last count putting one into
+// the next round.  The cells of a round are no neighbours of each other, so the result is the
+// sequential walk's exactly, and the rounds are as many as the longest chain of neighbouring cells:
+// 42 for a 160x192x160 field with 157,751 flagged cells, where a wavefront over the whole volume
+// (4x + 2y + z, one CTA) has 1,157 levels and took 3.1 ms; the rounds take 0.2 ms.
+struct LimiterArgs {
+    const uint8_t *mask;  // flagged corners of every cell (corner_kernel)
+    double *g;            // gradients [9][V]
+    int *deg;             // earlier flagged neighbours still to go, per cell
+    int *front[2];        // the cells of a round and of the next
+    int *counts;          // cells of each round
+    int nx, ny, nz;
+    double e1, e2;
+    unsigned *flags;
+};
+
+// neighbour q (0 .. 12) of the 13 that come later in lexicographic order: (dx, dy, dz) > 0
+__device__ __forceinline__ void later_neighbour(int q, int &dx, int &dy, int &dz) {
+    const int o = q + 14;  // 27 offsets in order, the cell itself is the 14th
+    dx = o / 9 - 1;
+    dy = o / 3 % 3 - 1;
+    dz = o % 3 - 1;
+}
+
+// The corners of one cell by a group of 16 lanes (gmask).  The 36 gradient entries its corners read
+// -- column n2 at the four vertices with coordinate n2 zero -- are loaded at once, entry i by lane
+// i % 16, and stay in the lanes until the end.  Per corner every lane gathers the 3x3 matrix; lane
+// t evaluates trial t of the limiter step (1 <= t <= 11, alpha `at`, the alpha after one step more
+// `an`), and the lowest lane whose determinant lies in [e1, e2] picks the step: limit_corner's
+// expressions and choice.
+__device__ __forceinline__ void limit_cell(const LimiterArgs &a, int x, int y, int z, unsigned mask,
+                                           int gl, unsigned gmask, double at, double an,
+                                           bool &capped) {
+    const long V = (long)a.nx * a.ny * a.nz;
+    double v[3];
+    double *src[3];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        const int i = gl + 16 * e;
+        if (i < 36) {
+            const int n2 = i / 12, n1 = i / 4 % 3, p = (i >> 1) & 1, q = i & 1;
+            const int ox = n2 == 0 ? 0 : p, oy = n2 == 0 ? p : (n2 == 1 ? 0 : q),
+                      oz = n2 == 2 ? 0 : q;
+            src[e] = a.g + (n1 * 3 + n2) * V + ((long)(x + ox) * a.ny + (y + oy)) * a.nz + (z + oz);
+            v[e] = *src[e];
+        } else {
+            src[e] = nullptr;
+            v[e] = 0.0;
+        }
     }
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int l = 0; l < nlev; ++l) off[l + 1] += off[l];
-    __syncthreads();
-    for (int l = threadIdx.x; l < nlev; l += blockDim.x) cur[l] = off[l];
-    __syncthreads();
-    for (int q = threadIdx.x; q < n; q += blockDim.x) {
-        const long cell = list[q];
-        const int x = (int)(cell / (cy * cz)), y = (int)((cell / cz) % cy), z = (int)(cell % cz);
-        sorted[atomicAdd(&cur[4 * x + 2 * y + z], 1)] = (int)cell;
+    constexpr int vert[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1},
+                                {0, 1, 1}, {1, 0, 1}, {1, 1, 0}, {1, 1, 1}};
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        if (!(mask >> c & 1u)) continue;  // uniform across the group
+        const int va = vert[c][0], vb = vert[c][1], vc = vert[c][2];
+        const int at0[3] = {vb * 2 + vc, va * 2 + vc, va * 2 + vb};
+        double J[3][3];
+#pragma unroll
+        for (int n1 = 0; n1 < 3; ++n1)
+#pragma unroll
+            for (int n2 = 0; n2 < 3; ++n2) {
+                const int i = (n2 * 3 + n1) * 4 + at0[n2];
+                J[n1][n2] = __shfl_sync(gmask, v[i >> 4], i & 15, 16);
+            }
+        const double det0 = detn<3>(J);
+        double alpha = 0.1;  // one step from 0
+        if (det0 > a.e2 || det0 < a.e1) {
+            bool in = false;
+            if (gl >= 1 && gl <= 11) {
+                double Jn[3][3];
+#pragma unroll
+                for (int n1 = 0; n1 < 3; ++n1)
+#pragma unroll
+                    for (int n2 = 0; n2 < 3; ++n2)
+                        Jn[n1][n2] = (1 - at) * J[n1][n2] + at * (n1 == n2 ? 1.0 : 0.0);
+                const double det = detn<3>(Jn);
+                in = !(det > a.e2 || det < a.e1);
+            }
+            const unsigned b = __ballot_sync(gmask, in) & gmask;
+            const int k = b ? __ffs((int)b) - 1 : -1;  // lane of the warp
+            alpha = __shfl_sync(gmask, an, k < 0 ? 11 : (k & 15), 16);  // al[k + 1], or al[12] = 1
+            if (k < 0) capped = true;
+        }
+#pragma unroll
+        for (int n1 = 0; n1 < 3; ++n1)
+#pragma unroll
+            for (int n2 = 0; n2 < 3; ++n2) {
+                const int i = (n2 * 3 + n1) * 4 + at0[n2];
+                const double w = (1 - alpha) * J[n1][n2] + alpha * (n1 == n2 ? 1.0 : 0.0);
+                if (gl == (i & 15)) v[i >> 4] = w;
+            }
     }
-    __syncthreads();
-    const int vert[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1},
-                            {0, 1, 1}, {1, 0, 1}, {1, 1, 0}, {1, 1, 1}};
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+        if (src[e]) *src[e] = v[e];
+}
+
+// the limiter's alphas after t steps and after t + 1 (0.1 at a time, capped at 1)
+__device__ __forceinline__ void trial_alphas(int t, double &at, double &an) {
+    at = 0.0;
+    for (int k = 0; k < t; ++k) {
+        at = at + 0.1;
+        if (at > 1.0) at = 1.0;
+    }
+    an = at + 0.1;
+    if (an > 1.0) an = 1.0;
+}
+
+// earlier flagged neighbours of a flagged cell
+__device__ __forceinline__ int earlier_flagged(const uint8_t *mask, int x, int y, int z, int cx,
+                                               int cy, int cz) {
+    int n = 0;
+#pragma unroll
+    for (int q = 0; q < 13; ++q) {
+        int dx, dy, dz;
+        later_neighbour(q, dx, dy, dz);
+        const int X = x - dx, Y = y - dy, Z = z - dz;
+        if (X >= 0 && Y >= 0 && Z >= 0 && X < cx && Y < cy && Z < cz)
+            n += mask[((long)X * cy + Y) * cz + Z] != 0;
+    }
+    return n;
+}
+
+// round 0: the flagged cells with no earlier flagged neighbour
+__global__ void limiter_start_kernel(const LimiterArgs a) {
+    const int cx = a.nx - 1, cy = a.ny - 1, cz = a.nz - 1;
+    const long cells = (long)cx * cy * cz;
+    for (long cell = (long)blockIdx.x * blockDim.x + threadIdx.x; cell < cells;
+         cell += (long)gridDim.x * blockDim.x) {
+        if (!a.mask[cell]) continue;
+        const int x = (int)(cell / ((long)cy * cz)), y = (int)((cell / cz) % cy),
+                  z = (int)(cell % cz);
+        const int n = earlier_flagged(a.mask, x, y, z, cx, cy, cz);
+        a.deg[cell] = n;
+        if (n == 0) a.front[0][atomicAdd(&a.counts[0], 1)] = (int)cell;
+    }
+}
+
+// one round over the whole GPU
+__global__ void __launch_bounds__(256) limiter_round_kernel(const LimiterArgs a, int round) {
+    const int n = a.counts[round];
+    const int gl = threadIdx.x & 15;
+    const unsigned gmask = 0xffffu << (threadIdx.x & 16);
+    const int cx = a.nx - 1, cy = a.ny - 1, cz = a.nz - 1;
+    const int *now = a.front[round & 1];
+    int *next = a.front[(round + 1) & 1];
+    double at, an;
+    trial_alphas(gl, at, an);
     bool capped = false;
-    for (int l = 0; l < nlev; ++l) {
-        const int beg = off[l], end = off[l + 1];
-        if (beg == end) continue;  // uniform: every thread reads the same shared value
-        for (int q = beg + threadIdx.x; q < end; q += blockDim.x) {
-            const long cell = sorted[q];
-            const int x = (int)(cell / (cy * cz)), y = (int)((cell / cz) % cy), z = (int)(cell % cz);
-            for (int c = 0; c < 8; ++c) {
-                const double jv = Jc[cell * 8 + c];
-                if (!(jv < e1 || jv > e2)) continue;
-                long gp[3];
-                for (int n2 = 0; n2 < 3; ++n2) {
-                    int o[3] = {vert[c][0], vert[c][1], vert[c][2]};
-                    o[n2] = 0;
-                    gp[n2] = ((long)(x + o[0]) * ny + (y + o[1])) * nz + (z + o[2]);
-                }
-                double J[3][3];
-                for (int n1 = 0; n1 < 3; ++n1)
-                    for (int n2 = 0; n2 < 3; ++n2) J[n1][n2] = g[(n1 * 3 + n2) * V + gp[n2]];
-                limit_corner<3>(J, e1, e2, capped);
-                for (int n1 = 0; n1 < 3; ++n1)
-                    for (int n2 = 0; n2 < 3; ++n2) g[(n1 * 3 + n2) * V + gp[n2]] = J[n1][n2];
+    for (int q = (blockIdx.x * 256 + threadIdx.x) >> 4; q < n; q += gridDim.x * 16) {
+        const long cell = now[q];
+        const int x = (int)(cell / ((long)cy * cz)), y = (int)((cell / cz) % cy),
+                  z = (int)(cell % cz);
+        limit_cell(a, x, y, z, a.mask[cell], gl, gmask, at, an, capped);
+        if (gl < 13) {
+            int dx, dy, dz;
+            later_neighbour(gl, dx, dy, dz);
+            const int X = x + dx, Y = y + dy, Z = z + dz;
+            if (X < cx && Y >= 0 && Y < cy && Z >= 0 && Z < cz) {
+                const long nb = ((long)X * cy + Y) * cz + Z;
+                if (a.mask[nb] && atomicSub(&a.deg[nb], 1) == 1)
+                    next[atomicAdd(&a.counts[round + 1], 1)] = (int)nb;
             }
         }
+        __syncwarp(gmask);
+    }
+    if (capped) atomicOr(a.flags, (unsigned)kFlagLimiterCapped);
+}
+
+// The rounds from `round` on, until none is left, in one CTA: small rounds cost less between two
+// barriers than as launches.  SM: a volume of at most kSmallCells cells, all rounds, with the masks,
+// counts and rounds in shared memory.
+constexpr int kSmallCells = 65536;
+constexpr int kTailThreads = 1024;
+template <bool SM>
+__global__ void __launch_bounds__(kTailThreads) limiter_tail_kernel(const LimiterArgs a, int round,
+                                                                    int cap) {
+    extern __shared__ __align__(16) unsigned char shm[];
+    __shared__ int cnt[2];
+    const int cx = a.nx - 1, cy = a.ny - 1, cz = a.nz - 1;
+    const int cells = SM ? cx * cy * cz : 0, words = (cells + 3) >> 2;
+    unsigned *deg = reinterpret_cast<unsigned *>(shm);                       // [words] 4 counts each
+    uint8_t *mask = reinterpret_cast<uint8_t *>(deg + words);                // [4 * words]
+    unsigned short *f16 = reinterpret_cast<unsigned short *>(mask + 4 * words);  // [2][cap]
+    const int tid = threadIdx.x, gl = tid & 15;
+    const unsigned gmask = 0xffffu << (tid & 16);
+    if (tid < 2) cnt[tid] = 0;
+    if (SM) {
+        for (int i = tid; i < 4 * words; i += kTailThreads) mask[i] = i < cells ? a.mask[i] : 0;
+        __syncthreads();
+        for (int w = tid; w < words; w += kTailThreads) {
+            unsigned d = 0;
+            for (int e = 0; e < 4; ++e) {
+                const int cell = 4 * w + e;
+                if (cell >= cells || !mask[cell]) continue;
+                const int x = cell / (cy * cz), y = cell / cz % cy, z = cell % cz;
+                const unsigned n = (unsigned)earlier_flagged(mask, x, y, z, cx, cy, cz);
+                d |= n << (8 * e);
+                if (n == 0) f16[atomicAdd(&cnt[0], 1)] = (unsigned short)cell;
+            }
+            deg[w] = d;
+        }
+    } else {
+        if (tid == 0) cnt[round & 1] = a.counts[round];
+    }
+    __syncthreads();
+    double at, an;
+    trial_alphas(gl, at, an);
+    bool capped = false;
+    for (;; ++round) {
+        const int cur = round & 1, n = cnt[cur];
+        if (n == 0) break;
+        for (int q = tid >> 4; q < n; q += kTailThreads / 16) {
+            const int cell = SM ? (int)f16[cur * cap + q] : a.front[cur][q];
+            const int x = cell / (cy * cz), y = cell / cz % cy, z = cell % cz;
+            limit_cell(a, x, y, z, SM ? mask[cell] : a.mask[cell], gl, gmask, at, an, capped);
+            if (gl < 13) {
+                int dx, dy, dz;
+                later_neighbour(gl, dx, dy, dz);
+                const int X = x + dx, Y = y + dy, Z = z + dz;
+                if (X < cx && Y >= 0 && Y < cy && Z >= 0 && Z < cz) {
+                    const int nb = (X * cy + Y) * cz + Z;
+                    if (SM) {
+                        const int sh = 8 * (nb & 3);
+                        if (mask[nb] && (atomicSub(&deg[nb >> 2], 1u << sh) >> sh & 0xffu) == 1u)
+                            f16[(cur ^ 1) * cap + atomicAdd(&cnt[cur ^ 1], 1)] = (unsigned short)nb;
+                    } else if (a.mask[nb] && atomicSub(&a.deg[nb], 1) == 1) {
+                        a.front[cur ^ 1][atomicAdd(&cnt[cur ^ 1], 1)] = nb;
+                    }
+                }
+            }
+            __syncwarp(gmask);
+        }
+        __syncthreads();  // the round's gradients and the next round are complete
+        if (tid == 0) cnt[cur] = 0;
         __syncthreads();
     }
-    if (capped) atomicOr(flags, (unsigned)kFlagLimiterCapped);
+    if (capped) atomicOr(a.flags, (unsigned)kFlagLimiterCapped);
+}
+
+// cells of a round at most: no two are neighbours
+int most_apart(int cx, int cy, int cz) {
+    return ((cx + 1) / 2) * ((cy + 1) / 2) * ((cz + 1) / 2);
+}
+
+constexpr int kMaxRounds = 24;  // rounds as launches of their own at most
+
+// the limiter over every flagged cell; `corners`: how many corners are flagged
+void launch_limiter(const LimiterArgs &a, long corners, cudaStream_t s) {
+    const int cx = a.nx - 1, cy = a.ny - 1, cz = a.nz - 1;
+    const long cells = (long)cx * cy * cz;
+    if (cells <= kSmallCells) {
+        const int cap = most_apart(cx, cy, cz);
+        const size_t smem = (size_t)(cells + 3) / 4 * 8 + (size_t)cap * 4;
+        BINDER_CUDA(cudaFuncSetAttribute(limiter_tail_kernel<true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        count_launch(), limiter_tail_kernel<true><<<1, kTailThreads, smem, s>>>(a, 0, cap);
+        BINDER_CUDA(cudaGetLastError());
+        return;
+    }
+    // the first rounds hold most of the cells of a field with many; a field with few is left to the
+    // one CTA
+    const int rounds = corners > 16384 ? kMaxRounds : (corners > 1024 ? 8 : 0);
+    BINDER_CUDA(cudaMemsetAsync(a.counts, 0, sizeof(int) * (kMaxRounds + 1), s));
+    long b = (cells + 255) / 256;
+    const int grid = (int)(b < 148L * 16 ? b : 148L * 16);
+    count_launch(), limiter_start_kernel<<<grid, 256, 0, s>>>(a);
+    b = (corners + 15) / 16;
+    const int rgrid = (int)(b < 148L * 8 ? b : 148L * 8);
+    for (int r = 0; r < rounds; ++r)
+        count_launch(), limiter_round_kernel<<<rgrid, 256, 0, s>>>(a, r);
+    count_launch(), limiter_tail_kernel<false><<<1, kTailThreads, 0, s>>>(a, rounds, 0);
+    BINDER_CUDA(cudaGetLastError());
 }
 
 // backward-difference divergence (periodic) of each component's gradient row; the reference's
@@ -941,16 +1142,28 @@ struct TopologyWorkspace::Impl {
     bool ready = false;
     DBuf<double> grad, jc, div, t1, t2;
     DBuf<int> list, sorted;
+    DBuf<uint8_t> mask;  // 3D: flagged corners per cell
+    DBuf<int> deg, counts;
     DBuf<int> slot;  // image node -> shared-memory slot of the 2D limiter, -1 between calls
-    DBuf<double> H[3], cs[3];
+    HartleyMatrix H[3];
+    DBuf<double> cs[3];
     Impl(int x, int y, int z, cudaStream_t s)
         : nx(x), ny(y), nz(z), N(z == 1 ? 2 : 3), V((long)x * y * z),
           cells(z == 1 ? (long)(x - 1) * (y - 1) : (long)(x - 1) * (y - 1) * (z - 1)), st(s),
           pos(V * N, s), red(1, s), flags(1, s) {}
+    ~Impl() {
+        for (auto &h : H) h.release(st);
+    }
     void ensure() {
         if (ready) return;
         grad.alloc(V * N * N, st);
-        jc.alloc(cells * (nz == 1 ? 4 : 8), st);
+        if (nz == 1) {
+            jc.alloc(cells * 4, st);
+        } else {
+            mask.alloc(cells, st);
+            deg.alloc(cells, st);
+            counts.alloc(kMaxRounds + 1, st);
+        }
         div.alloc(V * N, st);
         t1.alloc(V * N, st);
         t2.alloc(V * N, st);
@@ -964,16 +1177,13 @@ struct TopologyWorkspace::Impl {
         const double pi = 3.14159265358979323846;
         for (int a = 0; a < 3; ++a) {
             const int n = dims[a];
-            H[a].alloc((size_t)n * n, st);
+            H[a].init(n, st);
             cs[a].alloc(n, st);
-            std::vector<double> M((size_t)n * n), c(n);
-            hartley_matrix(n, M.data());
+            std::vector<double> c(n);
             for (int k = 0; k < n; ++k) c[k] = std::cos(2.0 * pi * k / (n * 1.0));
-            BINDER_CUDA(cudaMemcpyAsync(H[a].p, M.data(), sizeof(double) * n * n,
-                                        cudaMemcpyHostToDevice, st));
             BINDER_CUDA(cudaMemcpyAsync(cs[a].p, c.data(), sizeof(double) * n,
                                         cudaMemcpyHostToDevice, st));
-            BINDER_CUDA(cudaStreamSynchronize(st));  // the host tables go out of scope
+            BINDER_CUDA(cudaStreamSynchronize(st));  // `c` goes out of scope
         }
         ready = true;
     }
@@ -1009,8 +1219,8 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
     };
     auto corners = [&]() {
         reset_red(w.red.p, s);
-        count_launch(), corner_kernel<<<grid_for(cells), 256, 0, s>>>(w.pos.p, nx, ny, nz, vol, e1, e2, w.jc.p,
-                                                      w.red.p);
+        count_launch(), corner_kernel<<<grid_for(cells), 256, 0, s>>>(w.pos.p, nx, ny, nz, vol, e1, e2,
+                                                                      w.mask.p, w.red.p);
         BINDER_CUDA(cudaGetLastError());
         return read_red(w.red.p, s);
     };
@@ -1019,10 +1229,6 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
     double jmin = unordered(r.mn), jmax = unordered(r.mx);
     res.below_before = (long long)r.below;
     res.above_before = (long long)r.above;
-    const int nlev = 4 * (nx - 2) + 2 * (ny - 2) + (nz - 2) + 1;
-    const size_t lim_smem = sizeof(int) * (2 * (size_t)nlev + 1);
-    BINDER_CUDA(cudaFuncSetAttribute(limiter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)lim_smem));
     int outer = 0;
     while ((jmin < e1 || jmax > e2) && outer < max_outer) {
         w.ensure();
@@ -1032,10 +1238,17 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
             count_launch(), gradient_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, nx, ny, nz, vs[0], vs[1], vs[2],
                                                         w.grad.p);
             reset_red(w.red.p, s);
-            count_launch(), flag_cells_kernel<<<grid_for(cells), 256, 0, s>>>(w.jc.p, nx, ny, nz, e1, e2, w.list.p,
-                                                              w.red.p);
-            count_launch(), limiter_kernel<<<1, 256, lim_smem, s>>>(w.list.p, w.sorted.p, w.jc.p, w.grad.p, nx, ny,
-                                                     nz, e1, e2, nlev, w.red.p, w.flags.p);
+            LimiterArgs la{};
+            la.mask = w.mask.p;
+            la.g = w.grad.p;
+            la.deg = w.deg.p;
+            la.front[0] = w.list.p;
+            la.front[1] = w.sorted.p;
+            la.counts = w.counts.p;
+            la.nx = nx; la.ny = ny; la.nz = nz;
+            la.e1 = e1; la.e2 = e2;
+            la.flags = w.flags.p;
+            launch_limiter(la, (long)(c.below + c.above), s);
             BINDER_CUDA(cudaGetLastError());
             count_launch(), sum_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, V, 3, w.red.p);
             count_launch(), divergence_kernel<<<grid_for(V), 256, 0, s>>>(w.grad.p, nx, ny, nz, w.div.p);
@@ -1045,30 +1258,27 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
             for (int n = 0; n < 3; ++n) mean[n] = sr.sum[n] / (nx * ny * nz);
 
             // u = -(1/V) H (H div / lambda): separable Hartley passes z, y, [x fused], y, z
-            AxisArgs<double> a{};
-            a.comp_stride = V;
-            a.ny = ny;
+            HartleyArgs a{};
+            a.V = V;
             a.nz = nz;
             a.cos_x = w.cs[0].p;
             a.cos_y = w.cs[1].p;
             a.cos_z = w.cs[2].p;
-            a.in = w.div.p; a.out = w.t1.p; a.M = w.H[2].p; a.n = nz; a.outer = (long)nx * ny; a.s = 1;
-            launch_axis_pass(a, kEpiNone, 3, s);
-            a.in = w.t1.p; a.out = w.t2.p; a.M = w.H[1].p; a.n = ny; a.outer = nx; a.s = nz;
-            launch_axis_pass(a, kEpiNone, 3, s);
-            a.in = w.t2.p; a.out = w.t1.p; a.M = w.H[0].p; a.M2 = w.H[0].p; a.n = nx; a.outer = 1;
-            a.s = (long)ny * nz;
-            launch_axis_pass(a, kEpiPoisson, 3, s);
-            a.in = w.t1.p; a.out = w.t2.p; a.M = w.H[1].p; a.M2 = nullptr; a.n = ny; a.outer = nx;
-            a.s = nz;
-            launch_axis_pass(a, kEpiNone, 3, s);
+            a.in = w.div.p; a.out = w.t1.p; a.outer = (long)nx * ny; a.s = 1;
+            launch_hartley(a, w.H[2], kHartleyPlain, 3, s);
+            a.in = w.t1.p; a.out = w.t2.p; a.outer = nx; a.s = nz;
+            launch_hartley(a, w.H[1], kHartleyPlain, 3, s);
+            a.in = w.t2.p; a.out = w.t1.p; a.outer = 1; a.s = (long)ny * nz;
+            launch_hartley(a, w.H[0], kHartleyPoisson, 3, s);
+            a.in = w.t1.p; a.out = w.t2.p; a.outer = nx; a.s = nz;
+            launch_hartley(a, w.H[1], kHartleyPlain, 3, s);
             // last pass: physical positions u * vs + mean
-            a.in = w.t2.p; a.out = w.pos.p; a.M = w.H[2].p; a.n = nz; a.outer = (long)nx * ny; a.s = 1;
+            a.in = w.t2.p; a.out = w.pos.p; a.outer = (long)nx * ny; a.s = 1;
             for (int n = 0; n < 3; ++n) {
                 a.out_scale[n] = vs[n];
                 a.out_offset[n] = mean[n];
             }
-            launch_axis_pass(a, kEpiTopoOut, 3, s);
+            launch_hartley(a, w.H[2], kHartleyScaled, 3, s);
             c = corners();
             inner++;
             res.inner_iterations++;
@@ -1148,29 +1358,23 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
 
             // u = -(1/V) H (H div / lambda) on the nx x ny grid (the volume nx x ny x 1, whose
             // unit z axis contributes cos 0 = 1 to lambda = 6 - 2cos_x - 2cos_y - 2cos_z)
-            AxisArgs<double> a{};
-            a.comp_stride = V;
-            a.ny = ny;
+            HartleyArgs a{};
+            a.V = V;
             a.nz = 1;
             a.cos_x = w.cs[0].p;
             a.cos_y = w.cs[1].p;
             a.cos_z = w.cs[2].p;
-            a.in = w.div.p; a.out = w.t1.p; a.M = w.H[1].p; a.n = ny; a.outer = nx; a.s = 1;
-            launch_axis_pass(a, kEpiNone, 2, s);
-            // the x passes as two launches (forward with -1/lambda, inverse), each split into row
-            // blocks: fused into one, a 2D image's x pass fills only a few CTAs
-            a.in = w.t1.p; a.out = w.t2.p; a.M = w.H[0].p; a.n = nx; a.outer = 1; a.s = ny;
-            launch_axis_pass(a, kEpiPoissonFwd, 2, s);
-            a.in = w.t2.p; a.out = w.t1.p;
-            launch_axis_pass(a, kEpiNone, 2, s);
+            a.in = w.div.p; a.out = w.t1.p; a.outer = nx; a.s = 1;
+            launch_hartley(a, w.H[1], kHartleyPlain, 2, s);
+            a.in = w.t1.p; a.out = w.t2.p; a.outer = 1; a.s = ny;
+            launch_hartley(a, w.H[0], kHartleyPoisson, 2, s);
             // last pass: physical positions u * vs + mean
-            a.in = w.t1.p; a.out = w.pos.p; a.M = w.H[1].p; a.M2 = nullptr; a.n = ny; a.outer = nx;
-            a.s = 1;
+            a.in = w.t2.p; a.out = w.pos.p; a.outer = nx; a.s = 1;
             for (int n = 0; n < 2; ++n) {
                 a.out_scale[n] = vs[n];
                 a.out_offset[n] = mean[n];
             }
-            launch_axis_pass(a, kEpiTopoOut, 2, s);
+            launch_hartley(a, w.H[1], kHartleyScaled, 2, s);
             c = corners();
             inner++;
             res.inner_iterations++;

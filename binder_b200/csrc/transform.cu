@@ -1,4 +1,4 @@
-// Separable transform passes (DCT prior smoothing, Hartley Poisson solve) -- see transform.cuh.
+// Separable FP32 transform passes (DCT prior smoothing) -- see transform.cuh.
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -21,19 +21,10 @@ template <>
 struct Pitch<float> {
     static constexpr int v = 68;  // 16-byte aligned rows
 };
-template <>
-struct Pitch<double> {
-    static constexpr int v = 66;
-};
 
 __device__ __forceinline__ void load4(const float *p, float v[4]) {
     const float4 q = *reinterpret_cast<const float4 *>(p);
     v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-}
-__device__ __forceinline__ void load4(const double *p, double v[4]) {
-    const double2 a = *reinterpret_cast<const double2 *>(p);
-    const double2 b = *reinterpret_cast<const double2 *>(p + 2);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
 
 // acc[r][q] = sum_j M[k][j] * Xs[j][c] for rows k = k0 + ty + 16 r and columns c = 4 tx + q
@@ -70,30 +61,6 @@ __device__ __forceinline__ void gemm_tile(const T *__restrict__ M, int n, const 
 __device__ __forceinline__ float prior_normal(uint64_t seed, uint32_t i, uint32_t sweep,
                                               uint32_t chain, int comp) {
     return dct_prior_normal(seed, i, sweep, chain, comp);
-}
-
-// Hartley Poisson step of an x-axis pass (outer == 1, s == ny*nz) on rows k = k0 + ty + 16 r:
-// c <- -c / (lambda * V), lambda = 6 - 2cos z - 2cos x - 2cos y
-template <typename T, int R>
-__device__ __forceinline__ void poisson_scale(const AxisArgs<T> &a, T (&acc)[R][4], int k0,
-                                              long t0, int ncol, int tx, int ty) {
-    const int n = a.n, nz = a.nz;
-    const double inv_total = 1.0 / ((double)n * (double)a.s);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int k = k0 + ty + 16 * r;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = tx * 4 + q;
-            if (k < n && c < ncol) {
-                const long t = t0 + c;
-                const int ky = (int)(t / nz), kz = (int)(t - (long)ky * nz);
-                const double lam =
-                    6.0 - 2.0 * a.cos_z[kz] - 2.0 * a.cos_x[k] - 2.0 * a.cos_y[ky];
-                acc[r][q] = fabs(lam) > 1e-10 ? (T)(-(double)acc[r][q] / lam * inv_total) : T(0);
-            }
-        }
-    }
 }
 
 template <typename T, int R, int MODE>
@@ -155,12 +122,11 @@ __global__ void __launch_bounds__(kThreads) axis_kernel(const AxisArgs<T> a) {
 
     T acc[R][4];
     gemm_tile<T, R>(a.M, n, Xs, Ms, acc, tx, ty, k0);
-    if constexpr (MODE == kEpiPoissonFwd) poisson_scale<T, R>(a, acc, k0, t0, ncol, tx, ty);
 
-    if constexpr (MODE == kEpiSpectral || MODE == kEpiPoisson) {
+    if constexpr (MODE == kEpiSpectral) {
         // x-axis pass (outer == 1, s == ny*nz): coefficient (k, t) has flat index k*s + t
         double part_cost = 0.0, part_raw = 0.0;
-        if constexpr (MODE == kEpiSpectral) {
+        {
             const double g = st->gamma[cn];
             const float gs2 = (float)(g * a.sigma2);
             const uint32_t sweep = (uint32_t)st->sweep;
@@ -186,10 +152,8 @@ __global__ void __launch_bounds__(kThreads) axis_kernel(const AxisArgs<T> a) {
                     }
                 }
             }
-        } else {
-            poisson_scale<T, R>(a, acc, 0, t0, ncol, tx, ty);
         }
-        if constexpr (MODE == kEpiSpectral) {
+        {
             const double sc = block_sum(part_cost, red);
             if (threadIdx.x == 0) atomicAdd(&st->lp_tr, sc);
             if (a.want_raw) {  // uniform across the block: every thread takes the same branch
@@ -237,8 +201,6 @@ __global__ void __launch_bounds__(kThreads) axis_kernel(const AxisArgs<T> a) {
                                    : (cn == 1 ? (float)((i / a.nz) % a.ny) : (float)(i % a.nz));
                 }
                 val = (T)((float)val + xv);
-            } else if constexpr (MODE == kEpiTopoOut) {
-                val = (T)((double)val * a.out_scale[cn] + a.out_offset[cn]);
             }
             dst[e] = val;
         }
@@ -279,12 +241,6 @@ void launch_r(const AxisArgs<T> &a, int ncomp, cudaStream_t stream) {
 template <typename T, int MODE>
 void launch_mode(const AxisArgs<T> &a, int ncomp, cudaStream_t stream) {
     const int n = a.n;
-    if constexpr (std::is_same<T, double>::value &&
-                  (MODE == kEpiNone || MODE == kEpiTopoOut || MODE == kEpiPoissonFwd)) {
-        // FP64 passes of a small image fill a few CTAs: split the rows into 16-row blocks
-        const long gx = a.s == 1 ? (a.outer + TC - 1) / TC : a.outer * ((a.s + TC - 1) / TC);
-        if (n > 16 && gx * ncomp < 148) return launch_r<T, 1, MODE>(a, ncomp, stream);
-    }
     if (n <= 32)
         launch_r<T, 2, MODE>(a, ncomp, stream);
     else if (n <= 64)
@@ -305,27 +261,16 @@ void launch_axis_pass(const AxisArgs<T> &a, int mode, int ncomp, cudaStream_t st
     switch (mode) {
         case kEpiNone: launch_mode<T, kEpiNone>(a, ncomp, stream); break;
         case kEpiSpectral:
-            if constexpr (std::is_same<T, float>::value) launch_mode<T, kEpiSpectral>(a, ncomp, stream);
+            launch_mode<T, kEpiSpectral>(a, ncomp, stream);
             break;
         case kEpiPositions:
-            if constexpr (std::is_same<T, float>::value) launch_mode<T, kEpiPositions>(a, ncomp, stream);
-            break;
-        case kEpiPoisson:
-            if constexpr (std::is_same<T, double>::value) launch_mode<T, kEpiPoisson>(a, ncomp, stream);
-            break;
-        case kEpiTopoOut:
-            if constexpr (std::is_same<T, double>::value) launch_mode<T, kEpiTopoOut>(a, ncomp, stream);
-            break;
-        case kEpiPoissonFwd:
-            if constexpr (std::is_same<T, double>::value)
-                launch_mode<T, kEpiPoissonFwd>(a, ncomp, stream);
+            launch_mode<T, kEpiPositions>(a, ncomp, stream);
             break;
         default: BINDER_CHECK(false, "unknown transform epilogue");
     }
 }
 
 template void launch_axis_pass<float>(const AxisArgs<float> &, int, int, cudaStream_t);
-template void launch_axis_pass<double>(const AxisArgs<double> &, int, int, cudaStream_t);
 
 void dct2_matrix(int n, double *out) {
     // each size is built once per process (n^2 cosines: about 1.4 ms for the three axes of a
@@ -346,16 +291,6 @@ void dct2_matrix(int n, double *out) {
         }
     }
     std::copy(C.begin(), C.end(), out);
-}
-
-void hartley_matrix(int n, double *out) {
-    const double pi = 3.14159265358979323846;
-    for (int k = 0; k < n; ++k)
-        for (int j = 0; j < n; ++j) {
-            const long m = ((long)j * k) % n;
-            const double ang = 2.0 * pi * (double)m / n;
-            out[(long)k * n + j] = std::cos(ang) + std::sin(ang);
-        }
 }
 
 namespace {

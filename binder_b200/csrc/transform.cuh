@@ -31,10 +31,7 @@ enum EpilogueMode : int {
     kEpiNone = 0,       // plain store
     kEpiSpectral = 1,   // fused fwd -> DCT-prior scaling (+noise, costs) -> inverse (x axis)
     kEpiPositions = 2,  // store y + x_grid (final inverse pass) into the position field
-    kEpiPoisson = 3,    // fused fwd -> -1/lambda (Hartley Poisson) -> inverse (x axis)
-    kEpiTopoOut = 4,    // store u * scale + mean into a physical-position field (FP64)
     kEpiSpectralOut = 5,  // forward pass whose epilogue applies the prior scaling and stores it
-    kEpiPoissonFwd = 6,   // forward pass whose epilogue applies -1/lambda and stores it (FP64)
 };
 
 template <typename T>
@@ -65,10 +62,6 @@ struct AxisArgs {
     const float *xpos;  // SoA voxel positions or null for the identity grid
     int ny, nz;
     int dims;           // 3, or 2 for an nx x ny image (nz = 1, components x, y)
-    // Poisson epilogue: the periodic Laplacian symbol is 6 - 2cos_x - 2cos_y - 2cos_z
-    const double *cos_x, *cos_y, *cos_z;  // cos(2 pi k / n) per axis
-    double out_scale[3];   // kEpiTopoOut: per-component scale (voxel size / total)
-    double out_offset[3];  // kEpiTopoOut: per-component offset (mean)
     const int *skip;       // when non-null and *skip != 0 the pass is a no-op
     // a batch of chains: components chain * chain_comps + n (n < chain_comps) with states
     // st[chain] and Philox chain indices chain + chain; 0 for one chain
@@ -93,7 +86,5 @@ void launch_axis_pass(const AxisArgs<T> &a, int mode, int ncomp, cudaStream_t st
 
 // host-built orthonormal DCT-II matrix (rows = frequency) in double precision
 void dct2_matrix(int n, double *out);
-// host-built Hartley matrix cas(2 pi jk / n)
-void hartley_matrix(int n, double *out);
 
 }  // namespace binder
