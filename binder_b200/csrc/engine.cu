@@ -518,13 +518,13 @@ void Registration::load_bins(double alpha, const float *theta, int K, int L, int
     for (int m = 0; m < M; ++m)
         launch_bins_to_padded(bins + nv + m, w.nxn, w.nyn, w.nzn, K, vpad_ + padded * m, P_, Py,
                               PZ_, pyn_, zp_, M > 1 ? bad + 2 : bad + 1, s);
-    // the buffers of the order-independent histogram merge of the single-pass EM kernel (one
-    // channel, K <= 64)
-    if (M == 1 && K <= 64) {
-        hfix_ = dalloc<unsigned long long>((size_t)K * L, s);
+    // the buffers of the order-independent histogram merge of the single-pass EM kernels (one
+    // channel, K <= 64; the filter likelihood's column kernel)
+    if (M == 1 ? K <= 64 : filter_columns(K, L, M)) {
+        hfix_ = dalloc<unsigned long long>((size_t)cells, s);
         mpart_ = dalloc<double>(kEmPartials, s);
         BINDER_CUDA(cudaMemsetAsync(mpart_, 0, sizeof(double) * kEmPartials, s));
-        BINDER_CUDA(cudaMemsetAsync(hfix_, 0, sizeof(unsigned long long) * K * L, s));
+        BINDER_CUDA(cudaMemsetAsync(hfix_, 0, sizeof(unsigned long long) * cells, s));
     }
     BINDER_CUDA(cudaMemcpyAsync(theta_, theta, sizeof(float) * cells, cudaMemcpyDefault, s));
     BINDER_CUDA(cudaMemcpyAsync(theta0_, theta_, sizeof(float) * cells, cudaMemcpyDeviceToDevice, s));
@@ -752,7 +752,7 @@ void Registration::enqueue_em_iteration(int max_iter, double th, int update, cud
     else if (lk_ == 3)
         launch_ssdf_update(fst_, fstats_, update, st_, lk_stream_);
     else
-        launch_theta_update(theta_, hist_, lk_ == 2 ? nullptr : hfix_, mpart_, M_ * K_, L_, alpha_,
+        launch_theta_update(theta_, hist_, hfix_, mpart_, M_ * K_, L_, alpha_,
                             update, st_, lk_stream_);
     BINDER_CUDA(cudaEventRecord(lk_join_, lk_stream_));
     const double eta2[3] = {eta_[0] * eta_[0], eta_[1] * eta_[1], eta_[2] * eta_[2]};
@@ -1183,7 +1183,7 @@ double Registration::profile_stage(int stage, int n) {
         else if (lk_ == 3)
             launch_ssdf_update(fst_, fstats_, 0, st_, stream_);
         else
-            launch_theta_update(theta_, hist_, lk_ == 2 ? nullptr : hfix_, mpart_, M_ * K_, L_,
+            launch_theta_update(theta_, hist_, hfix_, mpart_, M_ * K_, L_,
                                 alpha_, 1, st_, stream_);
     };
     one();  // warm-up
@@ -1200,7 +1200,7 @@ double Registration::profile_stage(int stage, int n) {
     cudaEventDestroy(t1);
     BINDER_CUDA(cudaMemsetAsync(hist_, 0, sizeof(float) * M_ * K_ * L_, stream_));
     if (hfix_)
-        BINDER_CUDA(cudaMemsetAsync(hfix_, 0, sizeof(unsigned long long) * K_ * L_, stream_));
+        BINDER_CUDA(cudaMemsetAsync(hfix_, 0, sizeof(unsigned long long) * M_ * K_ * L_, stream_));
     BINDER_CUDA(cudaStreamSynchronize(stream_));
     return ms / n;
 }

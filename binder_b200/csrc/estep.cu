@@ -348,6 +348,29 @@ __device__ __forceinline__ void em_accumulate_log(const float *__restrict__ thu,
     mlog = m;
 }
 
+// The tail of a single-pass EM kernel: the CTA's fixed-point histogram [rows][LP] (rows x L cells)
+// into the global 64-bit sums, its log-likelihood into its partial (see estep_em_fast_kernel).
+template <int TPB>
+__device__ __forceinline__ void merge_cta(const EStepArgs &a, const unsigned *hs, int rows, int LP,
+                                          double mll, unsigned deg, double *red) {
+    const double m = block_sum(mll, red);
+    const double dg = block_sum((double)deg, red);
+    if (threadIdx.x == 0 && dg > 0.0) atomicAdd(&a.st->degenerate, (unsigned long long)dg);
+    const int L = a.L;
+    for (int q = threadIdx.x; q < rows * L; q += TPB) {
+        const int k = q / L;
+        const unsigned v = hs[k * LP + (q - k * L)];
+        if (v) atomicAdd(&a.hfix[q], (unsigned long long)v);
+    }
+    if (threadIdx.x == 0) {
+        a.mpart[blockIdx.x] = m;
+        if (blockIdx.x == 0) {
+            a.mpart[kMaxEmCtas] = a.hinv;
+            a.mpart[kMaxEmCtas + 1] = (double)gridDim.x;
+        }
+    }
+}
+
 // EM E-step for K <= 64 (BINDER/src/cpu/Registration.cpp:219-330, sample == false), one pass over
 // the 64 (3D) or 16 (2D) neighbours.  The posterior mass of a voxel is collected per moving bin k
 // in a private shared-memory column hk[k][thread] (bank = thread % 32, so never a conflict and
@@ -455,35 +478,12 @@ __global__ void __launch_bounds__(TPB, HC ? 3 : (TPB > kFastThreads ? 1 : 2))
         vp.store_r(a, i, V, fx + Sx * inv, fy + Sy * inv, fz + Sz * inv);
     }
     __syncthreads();
-    const double m = block_sum(mll, red);
-    const double dg = block_sum((double)deg, red);
-    if (threadIdx.x == 0 && dg > 0.0) atomicAdd(&a.st->degenerate, (unsigned long long)dg);
-    if (!a.hfix) {
-        for (int q = threadIdx.x; q < KL; q += TPB) {
-            const int k = q / L;
-            const unsigned v = hs[k * LP + (q - k * L)];
-            if (v) atomicAdd(&a.hist[q], (float)((double)v * a.hinv));
-        }
-        if (threadIdx.x == 0) atomicAdd(&a.st->mll, m);
-        return;
-    }
     // Order-independent merge, so that EM is bitwise repeatable: the CTA histograms are integers
     // and their 64-bit global sums are exact whatever order the CTAs arrive in.  The likelihood
     // update that follows on the stream converts the sums (one rounding per cell), clears them and
     // adds the CTAs' log-likelihood partials in CTA order (merged_cell, merge_mll).  Done here by
     // the last CTA to finish, it held up the M-step by 13 us whatever the volume.
-    for (int q = threadIdx.x; q < KL; q += TPB) {
-        const int k = q / L;
-        const unsigned v = hs[k * LP + (q - k * L)];
-        if (v) atomicAdd(&a.hfix[q], (unsigned long long)v);
-    }
-    if (threadIdx.x == 0) {
-        a.mpart[blockIdx.x] = m;
-        if (blockIdx.x == 0) {
-            a.mpart[kMaxEmCtas] = a.hinv;
-            a.mpart[kMaxEmCtas + 1] = (double)gridDim.x;
-        }
-    }
+    merge_cta<TPB>(a, hs, K, LP, mll, deg, red);
 }
 
 // Cell q of the joint histogram for the likelihood update: the FP32 histogram, plus what the
@@ -501,6 +501,131 @@ __device__ __forceinline__ void merge_mll(const double *mpart, DevState *st, dou
     for (unsigned b = threadIdx.x; b < n; b += blockDim.x) part += mpart[b];
     const double tot = block_sum(part, red);
     if (threadIdx.x == 0) st->mll += tot;
+}
+
+// EM E-step with the MI filter likelihood for up to four channels of up to 64 bins whose per-thread
+// bin columns fit in shared memory: the columns of estep_em_fast_kernel, one set per channel.  The
+// weight of a neighbour is its spline weight times prod_m theta[m][k_m][u_m]; it is added to every
+// channel's column, and the columns are flushed once per voxel as hist[m][k][u_m] += col / S in
+// fixed point.  Against two passes with one shared FP32 atomic (a compare-and-swap loop) per
+// neighbour and channel: 349 -> 79 us per launch at 64^3 with two channels of 48 bins.
+// Bound by the same issue and latency as the MI kernel, with as many warps as the columns leave.
+template <int DIM, int MC, int TPB>
+__global__ void __launch_bounds__(TPB, 1) estep_filter_col_kernel(const EStepArgs a) {
+    constexpr int Q = DIM == 3 ? 4 : 1;
+    if (a.skip && *a.skip) return;
+    extern __shared__ __align__(16) float sm[];
+    const int K = a.K, L = a.L, KL = K * L, K4 = (K + 3) & ~3;
+    const int KP = wide_pitch(K), LP = wide_pitch(L);
+    float *thT = sm;                                                        // [MC][L][KP]
+    unsigned *hs = reinterpret_cast<unsigned *>(sm + (size_t)MC * L * KP);  // [MC][K][LP]
+    float *cols = sm + (size_t)MC * (L * KP + K * LP);                      // [MC][K4][TPB]
+    __shared__ double red[32];
+#pragma unroll 4
+    for (int q = threadIdx.x; q < MC * KL; q += TPB) {
+        const int m = q / KL, e = q - m * KL, k = e / L, l = e - k * L;
+        thT[(m * L + l) * KP + k] = __ldg(a.theta + q);
+        hs[(m * K + k) * LP + l] = 0u;
+    }
+    for (int q = threadIdx.x; q < MC * K4 * TPB; q += TPB) cols[q] = 0.0f;
+    __syncthreads();
+    float *my = cols + threadIdx.x;  // channel m, bin k: my[(m * K4 + k) * TPB]
+    double mll = 0.0;
+    unsigned deg = 0;
+    const unsigned V = (unsigned)a.V, nz = (unsigned)a.nz, ny = (unsigned)a.ny;
+    for (unsigned i = blockIdx.x * TPB + threadIdx.x; i < V; i += gridDim.x * TPB) {
+        VoxelPos<DIM> vp;
+        if (!vp.load(a, i, V, ny, nz)) {
+            vp.store_r(a, i, V, vp.px, vp.py, vp.pz);
+            ++deg;
+            continue;
+        }
+        float bx[4], by[4] = {1.f, 1.f, 1.f, 1.f}, bz[4];
+        const int ix = spline_setup(vp.px, a.order, bx);
+        const int iy = DIM == 3 ? spline_setup(vp.py, a.order, by) : 0;
+        const int iz = spline_setup(vp.pz, a.order, bz);
+        const float fx = (float)ix, fy = (float)iy, fz = (float)iz;
+        int um[MC], lo[MC], hi[MC];
+        unsigned tha[MC];
+#pragma unroll
+        for (int m = 0; m < MC; ++m) {
+            um[m] = a.u[m * a.uch + i];
+            tha[m] = (unsigned)__cvta_generic_to_shared(thT + (m * L + um[m]) * KP);
+            lo[m] = 255;
+            hi[m] = 0;
+        }
+        float S = 0.0f, Sx = 0.0f, Sy = 0.0f, Sz = 0.0f;
+#pragma unroll 1
+        for (int p = 0; p < 4; ++p) {
+            // the plane's bins of every channel first, all loads in flight
+            uint32_t w[MC][Q];
+#pragma unroll
+            for (int m = 0; m < MC; ++m)
+#pragma unroll
+                for (int q = 0; q < Q; ++q)
+                    w[m][q] = gather_word<DIM>(a, a.vpad + m * a.vch, ix, iy, iz, p, q);
+            const float bxp = p == 0 ? bx[0] : (p == 1 ? bx[1] : (p == 2 ? bx[2] : bx[3]));
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const float bxy = Q == 4 ? bxp * by[q] : bxp;
+                float t[4] = {bxy * bz[0], bxy * bz[1], bxy * bz[2], bxy * bz[3]};
+#pragma unroll
+                for (int m = 0; m < MC; ++m)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        float th;
+                        asm("ld.shared.f32 %0, [%1];"
+                            : "=f"(th)
+                            : "r"(__dp4a(w[m][q], 4u << (8 * c), tha[m])));
+                        t[c] *= th;
+                    }
+                const float s4 = (t[0] + t[1]) + (t[2] + t[3]);
+                S += s4;
+                Sx += (float)(p - 1) * s4;
+                if (Q == 4) Sy += (float)(q - 1) * s4;
+                Sz += (t[2] - t[0]) + 2.0f * t[3];
+#pragma unroll
+                for (int m = 0; m < MC; ++m) {
+                    const uint32_t word = w[m][q];
+                    const int k0 = word & 0xff, k1 = (word >> 8) & 0xff, k2 = (word >> 16) & 0xff,
+                              k3 = word >> 24;
+                    float *col = my + (size_t)m * K4 * TPB;
+                    col_add2<TPB>(col, k0, k1, make_float2(t[0], t[1]));
+                    col_add2<TPB>(col, k2, k3, make_float2(t[2], t[3]));
+                    lo[m] = min(min(lo[m], min(k0, k1)), min(k2, k3));
+                    hi[m] = max(max(hi[m], max(k0, k1)), max(k2, k3));
+                }
+            }
+        }
+        const bool ok = S > 0.0f;
+        const float inv = ok ? 1.0f / S : 0.0f;
+        const float invs = inv * a.hscale;
+#pragma unroll
+        for (int m = 0; m < MC; ++m) {
+            unsigned *hcol = hs + (size_t)m * K * LP + um[m];
+            float *col = my + (size_t)m * K4 * TPB;
+            for (int k = lo[m] & ~3; k <= hi[m]; k += 4) {
+                float v[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = col[(k + e) * TPB];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (ok && v[e] != 0.0f)
+                        atomicAdd(&hcol[(k + e) * LP], __float2uint_rn(v[e] * invs));
+                    col[(k + e) * TPB] = 0.0f;
+                }
+            }
+        }
+        if (!ok) {
+            vp.store_r(a, i, V, fx, fy, fz);
+            ++deg;
+            continue;
+        }
+        mll -= (double)logf(S);
+        vp.store_r(a, i, V, fx + Sx * inv, fy + Sy * inv, fz + Sz * inv);
+    }
+    __syncthreads();
+    merge_cta<TPB>(a, hs, MC * K, LP, mll, deg, red);
 }
 
 // EM E-step with the MI filter likelihood (BINDER/src/cpu/MILikelihoodFilter.cpp:53-68 and
@@ -1603,6 +1728,35 @@ const void *estep_fn(bool sample, int K, bool logt, bool half, bool wide) {
                                   : (const void *)estep_kernel<false, DIM>);
 }
 
+// threads of the filter likelihood's column kernel: the most (of 512, 384, 256) whose columns fit
+// beside the tables, 0: it does not take this likelihood
+int filter_col_threads(int K, int L, int M) {
+    if (M > 4 || K > kSmallK) return 0;
+    const size_t tables = (size_t)M * (L * wide_pitch(K) + K * wide_pitch(L)) * sizeof(float);
+    for (int t : {512, 384, 256})
+        if (tables + (size_t)M * ((K + 3) & ~3) * t * sizeof(float) + 512 <= 227 * 1024) return t;
+    return 0;
+}
+size_t filter_col_smem(int K, int L, int M, int tpb) {
+    return ((size_t)M * (L * wide_pitch(K) + K * wide_pitch(L)) +
+            (size_t)M * ((K + 3) & ~3) * tpb) * sizeof(float);
+}
+template <int DIM, int MC>
+const void *filter_col_fn_m(int tpb) {
+    if (tpb == 512) return (const void *)estep_filter_col_kernel<DIM, MC, 512>;
+    if (tpb == 384) return (const void *)estep_filter_col_kernel<DIM, MC, 384>;
+    return (const void *)estep_filter_col_kernel<DIM, MC, 256>;
+}
+template <int DIM>
+const void *filter_col_fn(int M, int tpb) {
+    switch (M) {
+        case 1: return filter_col_fn_m<DIM, 1>(tpb);
+        case 2: return filter_col_fn_m<DIM, 2>(tpb);
+        case 3: return filter_col_fn_m<DIM, 3>(tpb);
+        default: return filter_col_fn_m<DIM, 4>(tpb);
+    }
+}
+
 size_t filter_smem(int K, int L, int M, bool sample = false) {
     return ((size_t)M * (L * theta_pitch(K) + K * theta_pitch(L)) + (sample ? 16 * kEThreads : 0)) *
            sizeof(float);
@@ -1643,6 +1797,7 @@ void launch_ssdf_dim(const EStepArgs &a, bool sample, int grid, size_t smem, cud
         launch_ssdf_dim_s<DIM, false>(a, grid, smem, s);
 }
 
+constexpr int kFilterPasses = 0;  // `ftpb` of the filter likelihood's two-pass kernel
 template <int DIM>
 void launch_estep_dim(const EStepArgs &a, bool sample, int grid, size_t smem, cudaStream_t s,
                       int ftpb) {
@@ -1650,7 +1805,12 @@ void launch_estep_dim(const EStepArgs &a, bool sample, int grid, size_t smem, cu
         launch_ssdf_dim<DIM>(a, sample, grid, smem, s);
     else if (a.filter && sample)
         count_launch(), estep_filter_kernel<DIM, true><<<grid, kEThreads, smem, s>>>(a);
-    else if (a.filter)
+    else if (a.filter && ftpb != kFilterPasses) {
+        void *args[] = {const_cast<EStepArgs *>(&a)};
+        count_launch();
+        BINDER_CUDA(cudaLaunchKernel(filter_col_fn<DIM>(a.M, ftpb), dim3((unsigned)grid),
+                                     dim3((unsigned)ftpb), args, smem, s));
+    } else if (a.filter)
         count_launch(), estep_filter_kernel<DIM><<<grid, kEThreads, smem, s>>>(a);
     else if (a.logt && sample)
         count_launch(), estep_kernel<true, DIM, true><<<grid, kEThreads, smem, s>>>(a);
@@ -1699,6 +1859,8 @@ int estep_grid(bool sample, int K, int L, long V, int dim, bool logt, bool half)
     return (int)g;
 }
 
+bool filter_columns(int K, int L, int M) { return filter_col_threads(K, L, M) > 0; }
+
 bool filter_sampling_fits(int K, int L, int M) {
     return filter_smem(K, L, M, true) <= 227 * 1024;
 }
@@ -1710,6 +1872,17 @@ int estep_filter_grid(int K, int L, int M, long V, int dim, bool sample) {
     int dev = 0, sms = 148, per_sm = 1;
     BINDER_CUDA(cudaGetDevice(&dev));
     BINDER_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (const int t = sample ? 0 : filter_col_threads(K, L, M)) {
+        const void *fn = dim == 3 ? filter_col_fn<3>(M, t) : filter_col_fn<2>(M, t);
+        BINDER_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)filter_col_smem(K, L, M, t)));
+        BINDER_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         (int)cudaSharedmemCarveoutMaxShared));
+        BINDER_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, fn, t, filter_col_smem(K, L, M, t)));
+        const long need = (V + t - 1) / t, g = (long)sms * (per_sm < 1 ? 1 : per_sm);
+        return (int)(need < g ? (need < 1 ? 1 : need) : g);
+    }
     const size_t smem = filter_smem(K, L, M, sample);
     BINDER_CHECK(smem <= 227 * 1024,
                  sample ? "the MI filter likelihood's theta, counts and draw table do not fit in "
@@ -1789,12 +1962,15 @@ void launch_estep(const EStepArgs &args, bool sample, int grid, cudaStream_t s, 
     EStepArgs a = args;
     if (sample || a.logt || a.filter || a.ssdf) a.halfcol = 0;  // FP32 columns only there
     // threads per CTA of the single-pass EM kernel (the same choice as estep_grid's)
-    const int ftpb = (sample || a.filter || a.ssdf)
+    const int ftpb = a.filter && !sample ? (a.hfix ? filter_col_threads(a.K, a.L, a.M) : kFilterPasses)
+                     : (sample || a.ssdf)
                          ? kFastThreads
                          : fast_threads(a.V, a.K, a.L, a.logt != 0, a.halfcol != 0);
     a.tpitch = general_pitch(a.K, a.L, sample);
     const size_t smem = a.ssdf     ? ssdf_smem(a.M, a.Fn, sample)
-                        : a.filter ? filter_smem(a.K, a.L, a.M, sample)
+                        : a.filter ? (ftpb != kFilterPasses && !sample
+                                          ? filter_col_smem(a.K, a.L, a.M, ftpb)
+                                          : filter_smem(a.K, a.L, a.M, sample))
                                    : estep_smem(sample, a.K, a.L, a.logt != 0, a.halfcol != 0,
                                                 ftpb);
     // the order-independent merge of the single-pass EM kernel keeps one partial per CTA
@@ -1803,7 +1979,8 @@ void launch_estep(const EStepArgs &args, bool sample, int grid, cudaStream_t s, 
     // which the voxels one CTA visits, each adding at most scale + 1/2 (a posterior of 1, rounded;
     // FP32 rounding of m / S can exceed 1 by a few ulps, covered by the factor 1 + 2^-16) to a
     // cell, fit in 32 bits
-    const long per_cta = ((a.V + (long)grid * ftpb - 1) / ((long)grid * ftpb)) * ftpb;
+    const long tpb = ftpb > 0 ? ftpb : kEThreads;
+    const long per_cta = ((a.V + (long)grid * tpb - 1) / ((long)grid * tpb)) * tpb;
     double sc = std::floor(4294967295.0 / ((double)per_cta * (1.0 + 1.0 / 65536.0)) - 1.0);
     sc = sc < 1.0 ? 1.0 : (sc > 1073741824.0 ? 1073741824.0 : sc);
     float fsc = (float)sc;

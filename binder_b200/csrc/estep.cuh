@@ -81,6 +81,9 @@ constexpr int kLogMaxBins = 64;
 constexpr int kMaxChannels = 8;
 constexpr long kFilterMaxCells = 24576;
 int estep_filter_grid(int K, int L, int M, long V, int dim, bool sample = false);
+// whether the EM E-step of the MI filter likelihood keeps bin columns (it then needs
+// EStepArgs::hfix / mpart)
+bool filter_columns(int K, int L, int M);
 // whether the sampling E-step of the MI filter likelihood fits in shared memory (theta, counts
 // and its per-thread draw table)
 bool filter_sampling_fits(int K, int L, int M);
