@@ -95,6 +95,34 @@ void replay(const Graph &graph, long long kernels, cudaStream_t s) {
     count_launch(kernels);
 }
 
+// Branches of a captured graph without a stream per branch: the nodes that the next captured
+// node of stream s follows are read, replaced and joined directly (a second stream costs 0.1 ms
+// to make and give back, for every registration object).  Without a capture under way the three
+// do nothing and the work runs in stream order.
+using GraphTail = std::vector<cudaGraphNode_t>;
+
+GraphTail graph_tail(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t *nodes = nullptr;
+    size_t n = 0;
+    BINDER_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &nodes, &n));
+    return status == cudaStreamCaptureStatusActive ? GraphTail(nodes, nodes + n) : GraphTail();
+}
+
+void update_graph_tail(cudaStream_t s, const GraphTail &t, unsigned flags) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    BINDER_CUDA(cudaStreamGetCaptureInfo(s, &status));
+    if (status != cudaStreamCaptureStatusActive) return;
+    GraphTail nodes = t;
+    BINDER_CUDA(cudaStreamUpdateCaptureDependencies(s, nodes.data(), nodes.size(), flags));
+}
+void set_graph_tail(cudaStream_t s, const GraphTail &t) {
+    update_graph_tail(s, t, cudaStreamSetCaptureDependencies);
+}
+void add_graph_tail(cudaStream_t s, const GraphTail &t) {
+    update_graph_tail(s, t, cudaStreamAddCaptureDependencies);
+}
+
 }  // namespace
 
 void EmGraphCache::clear() {
@@ -113,43 +141,62 @@ long long &launch_counter() {
 // ------------------------------------------------------------------------------------------
 void DctSet::init(int nx, int ny, int nz, cudaStream_t s) {
     const int dims[3] = {nx, ny, nz};
-    for (int a = 0; a < 3; ++a) {
-        const int m = dims[a];
-        n[a] = m;
-        // the unit z axis of a 2D image has no transform; a unit axis of the image itself has
-        // the 1 x 1 identity
-        if (a == 2 && nz == 1) continue;
-        std::vector<double> C((size_t)m * m);
-        dct2_matrix(m, C.data());
-        std::vector<float> F((size_t)m * m), I((size_t)m * m);
-        for (int k = 0; k < m; ++k)
-            for (int j = 0; j < m; ++j) {
-                F[(size_t)k * m + j] = (float)C[(size_t)k * m + j];
-                I[(size_t)j * m + k] = (float)C[(size_t)k * m + j];
-            }
-        fwd[a] = dalloc<float>((size_t)m * m, s);
-        inv[a] = dalloc<float>((size_t)m * m, s);
-        std::vector<double> CT((size_t)m * m);
-        for (int k = 0; k < m; ++k)
-            for (int j = 0; j < m; ++j) CT[(size_t)j * m + k] = C[(size_t)k * m + j];
-        ufwd[a].init(C.data(), m, s);
-        uinv[a].init(CT.data(), m, s);
-        BINDER_CUDA(cudaMemcpyAsync(fwd[a], F.data(), sizeof(float) * m * m,
-                                    cudaMemcpyHostToDevice, s));
-        BINDER_CUDA(cudaMemcpyAsync(inv[a], I.data(), sizeof(float) * m * m,
-                                    cudaMemcpyHostToDevice, s));
-        BINDER_CUDA(cudaStreamSynchronize(s));  // F and I go out of scope
+    const int axes = nz == 1 ? 2 : 3;  // the unit z axis of a 2D image has no transform; a unit
+                                       // axis of the image itself has the 1 x 1 identity
+    // one buffer: the matrices of the distinct lengths (the part that is uploaded), then what
+    // the device derives from them.  Every piece starts on a 256-byte boundary.
+    auto aligned = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    int same[3];  // the first axis of the same length
+    size_t mat[3], upload = 0;
+    for (int a = 0; a < axes; ++a) {
+        n[a] = dims[a];
+        same[a] = a;
+        for (int b = a - 1; b >= 0; --b)
+            if (dims[b] == dims[a]) same[a] = b;
+        mat[a] = upload;
+        if (same[a] == a) upload += aligned(sizeof(float) * dims[a] * dims[a]);
     }
+    size_t total = upload;
+    for (int a = 0; a < axes; ++a)
+        if (same[a] == a)
+            total += aligned(sizeof(float) * dims[a] * dims[a]) +
+                     2 * aligned(sizeof(float) * UmmaMatrix::elements(dims[a])) +
+                     2 * aligned(sizeof(uint16_t) * UmmaMatrix::elements(dims[a]));
+    buf = dalloc<unsigned char>(total, s);
+    std::vector<unsigned char> host(upload);
+    for (int a = 0; a < axes; ++a) {
+        if (same[a] != a) continue;
+        const std::vector<double> &C = dct2_matrix(dims[a]);
+        float *F = reinterpret_cast<float *>(host.data() + mat[a]);
+        for (size_t i = 0; i < C.size(); ++i) F[i] = (float)C[i];
+    }
+    BINDER_CUDA(cudaMemcpyAsync(buf, host.data(), upload, cudaMemcpyHostToDevice, s));
+    size_t at = upload;
+    auto take = [&](size_t bytes) {
+        unsigned char *p = buf + at;
+        at += aligned(bytes);
+        return p;
+    };
+    for (int a = 0; a < axes; ++a) {
+        const int m = dims[a];
+        if (same[a] != a) {
+            fwd[a] = fwd[same[a]], inv[a] = inv[same[a]];
+            ufwd[a] = ufwd[same[a]], uinv[a] = uinv[same[a]];
+            continue;
+        }
+        const size_t ne = UmmaMatrix::elements(m);
+        fwd[a] = reinterpret_cast<float *>(buf + mat[a]);
+        inv[a] = reinterpret_cast<float *>(take(sizeof(float) * m * m));
+        for (UmmaMatrix *u : {&ufwd[a], &uinv[a]}) {
+            float *planes = reinterpret_cast<float *>(take(sizeof(float) * ne));
+            u->attach(m, planes, reinterpret_cast<uint16_t *>(take(sizeof(uint16_t) * ne)));
+        }
+        launch_format_matrix(fwd[a], inv[a], ufwd[a], uinv[a], s);
+    }
+    BINDER_CUDA(cudaStreamSynchronize(s));  // `host` goes out of scope
 }
 
-void DctSet::release(cudaStream_t s) {
-    for (int a = 0; a < 3; ++a) {
-        dfree(fwd[a], s);
-        dfree(inv[a], s);
-        ufwd[a].release(s);
-        uinv[a].release(s);
-    }
-}
+void DctSet::release(cudaStream_t s) { dfree(buf, s); }
 
 void MStep::init(int x, int y, int z, cudaStream_t s, int nchains) {
     nx = x; ny = y; nz = z;
@@ -167,11 +214,16 @@ void MStep::init(int x, int y, int z, cudaStream_t s, int nchains) {
         const bool off = e && e[0] == '0' && e[1] == 0;
         fused2d = chains == 1 && !off && z == 1 && x <= kM2dMaxN && y <= kM2dMaxN;
     }
+}
+
+// the streams of the per-component branches, made by the first M-step that takes them (a stream
+// costs 0.1 ms to make and give back, and the paired passes need none)
+void MStep::make_branches() {
     for (int i = 0; i < 2; ++i) {
-        BINDER_CUDA(cudaStreamCreate(&side[i]));
-        BINDER_CUDA(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming));
+        if (!side[i]) BINDER_CUDA(cudaStreamCreate(&side[i]));
+        if (!join[i]) BINDER_CUDA(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming));
     }
-    BINDER_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    if (!fork) BINDER_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
 }
 
 bool default_persistent() {
@@ -263,8 +315,9 @@ void MStep::enqueue(const float *r, float *d, const float *xpos, const float *D,
         return;
     }
     // the tensor-core path runs one chain of passes per component, each on its own stream
-    const bool branches = tc && !persistent && side[0] && side[1];
+    const bool branches = tc && !persistent;
     if (branches) {
+        make_branches();
         BINDER_CUDA(cudaEventRecord(fork, s));
         for (int c = 1; c < ncomp; ++c) BINDER_CUDA(cudaStreamWaitEvent(side[c - 1], fork, 0));
         for (int c = 0; c < ncomp; ++c)
@@ -410,9 +463,6 @@ Registration::Registration(const float *final_locations, const float *voxel_pos,
     // dream locations start at zero: r = 0 - x
     launch_aos_minus_to_soa(nullptr, x_, g, r_, s);
     mstep_.init(nx, ny, nz, s);
-    BINDER_CUDA(cudaStreamCreate(&lk_stream_));
-    BINDER_CUDA(cudaEventCreateWithFlags(&lk_fork_, cudaEventDisableTiming));
-    BINDER_CUDA(cudaEventCreateWithFlags(&lk_join_, cudaEventDisableTiming));
     BINDER_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -420,9 +470,6 @@ Registration::~Registration() {
     // nothing of this object may still run when its buffers go back to the pool
     if (stream_ != own_stream_) cudaStreamSynchronize(stream_);
     cudaStreamSynchronize(own_stream_);
-    if (lk_stream_) cudaStreamSynchronize(lk_stream_), cudaStreamDestroy(lk_stream_);
-    if (lk_fork_) cudaEventDestroy(lk_fork_);
-    if (lk_join_) cudaEventDestroy(lk_join_);
     em_graph_.clear();
     const cudaStream_t s = own_stream_;
     dfree(d_, s); dfree(x_, s); dfree(r_, s); dfree(D_, s); dfree(theta_, s); dfree(hist_, s);
@@ -743,22 +790,23 @@ void Registration::enqueue_em_iteration(int max_iter, double th, int update, cud
     const int grid = estep_grid_override_ > 0 ? estep_grid_override_ : egrid_e_;
     launch_estep(estep_args(&st_->done), false, grid, s);
     // the likelihood update (one CTA) reads the E-step's histogram or statistics and the M-step
-    // the dream locations: the two run side by side and join before the bookkeeping
-    BINDER_CUDA(cudaEventRecord(lk_fork_, s));
-    BINDER_CUDA(cudaStreamWaitEvent(lk_stream_, lk_fork_, 0));
+    // the dream locations: the two are branches of the captured graph and join before the
+    // bookkeeping
+    const GraphTail fork = graph_tail(s);
     if (lk_ == 1)
         launch_ssd_update(theta_, colmax_, hist_, hfix_, mpart_, K_, L_, update, ssd_, st_,
-                          lk_stream_);
+                          s);
     else if (lk_ == 3)
-        launch_ssdf_update(fst_, fstats_, update, st_, lk_stream_);
+        launch_ssdf_update(fst_, fstats_, update, st_, s);
     else
         launch_theta_update(theta_, hist_, hfix_, mpart_, M_ * K_, L_, alpha_,
-                            update, st_, lk_stream_);
-    BINDER_CUDA(cudaEventRecord(lk_join_, lk_stream_));
+                            update, st_, s);
+    const GraphTail likelihood = graph_tail(s);
+    set_graph_tail(s, fork);
     const double eta2[3] = {eta_[0] * eta_[0], eta_[1] * eta_[1], eta_[2] * eta_[2]};
     mstep_.enqueue(r_, d_, x_, D_, st_, sigma2_, 0, 0, 1, seed_, chain_,
                    rho_[0] * rho_[1] * rho_[2], eta2, &st_->done, s);
-    BINDER_CUDA(cudaStreamWaitEvent(s, lk_join_, 0));
+    add_graph_tail(s, likelihood);
     launch_em_finish(st_, stats_, max_iter, th, nzv_, s);
 }
 
@@ -1349,24 +1397,12 @@ RegistrationBatch::RegistrationBatch(const std::vector<Registration *> &regs) : 
     BINDER_CHECK(!regs.empty(), "a batch needs at least one registration");
     for (auto *r : regs) BINDER_CHECK(r != nullptr, "a batch member is null");
     BINDER_CUDA(cudaStreamCreateWithFlags(&master_, cudaStreamNonBlocking));
-    BINDER_CUDA(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
-    branch_.resize(regs.size(), nullptr);
-    join_.resize(regs.size(), nullptr);
     BINDER_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&done_host_), sizeof(int) * regs.size(),
                               cudaHostAllocDefault));
-    for (size_t i = 0; i < regs.size(); ++i) {
-        BINDER_CUDA(cudaStreamCreateWithFlags(&branch_[i], cudaStreamNonBlocking));
-        BINDER_CUDA(cudaEventCreateWithFlags(&join_[i], cudaEventDisableTiming));
-    }
 }
 
 RegistrationBatch::~RegistrationBatch() {
     if (master_) cudaStreamSynchronize(master_);
-    for (size_t i = 0; i < branch_.size(); ++i) {
-        if (branch_[i]) cudaStreamSynchronize(branch_[i]), cudaStreamDestroy(branch_[i]);
-        if (join_[i]) cudaEventDestroy(join_[i]);
-    }
-    if (fork_) cudaEventDestroy(fork_);
     if (master_) cudaStreamDestroy(master_);
     if (done_host_) cudaFreeHost(done_host_);
 }
@@ -1385,13 +1421,16 @@ void RegistrationBatch::em(int max_iterations, double th, int update, int *its_o
     for (size_t i = 0; i < active.size(); ++i) active[i] = i;
     Graph graph;
     const long long kernels = capture_graph(master_, graph, [&] {
-        BINDER_CUDA(cudaEventRecord(fork_, master_));
-        for (size_t i = 0; i < regs_.size(); ++i) {
-            BINDER_CUDA(cudaStreamWaitEvent(branch_[i], fork_, 0));
-            regs_[i]->enqueue_em(1, max_iterations, th, update, branch_[i]);
-            BINDER_CUDA(cudaEventRecord(join_[i], branch_[i]));
-            BINDER_CUDA(cudaStreamWaitEvent(master_, join_[i], 0));
+        // every pair is a branch of its own
+        const GraphTail root = graph_tail(master_);
+        GraphTail ends;
+        for (auto *r : regs_) {
+            set_graph_tail(master_, root);
+            r->enqueue_em(1, max_iterations, th, update, master_);
+            const GraphTail end = graph_tail(master_);
+            ends.insert(ends.end(), end.begin(), end.end());
         }
+        set_graph_tail(master_, ends);
     });
     cudaEvent_t t0, t1;
     BINDER_CUDA(cudaEventCreate(&t0));

@@ -16,6 +16,7 @@ struct DctSet {
     float *fwd[3] = {nullptr, nullptr, nullptr};
     float *inv[3] = {nullptr, nullptr, nullptr};
     UmmaMatrix ufwd[3], uinv[3];  // the same matrices preformatted for the tensor cores
+    unsigned char *buf = nullptr;  // all of them (axes of equal length share theirs)
     void init(int nx, int ny, int nz, cudaStream_t s);
     void release(cudaStream_t s);
 };
@@ -47,6 +48,7 @@ struct MStep {
     // buffers from the stream-ordered pool on stream s
     void init(int nx, int ny, int nz, cudaStream_t s, int chains = 1);
     void prepare_sampling(cudaStream_t s);
+    void make_branches();
     void release(cudaStream_t s);
     void enqueue(const float *r, float *d, const float *xpos, const float *D, DevState *st,
                  double sigma2, int sample, int want_raw, int every, uint64_t seed, uint32_t chain,
@@ -193,9 +195,6 @@ class Registration {
     // own_stream_ owns the buffers (pool allocations and frees); stream_ (own_stream_ unless the
     // caller set one) carries the copies and kernels
     cudaStream_t stream_ = 0, own_stream_ = 0;
-    // the likelihood update of an EM iteration runs on lk_stream_, beside the M-step
-    cudaStream_t lk_stream_ = nullptr;
-    cudaEvent_t lk_fork_ = nullptr, lk_join_ = nullptr;
     uint32_t chain_ = 0;
     // device buffers
     float *d_ = nullptr, *x_ = nullptr, *r_ = nullptr, *D_ = nullptr, *theta_ = nullptr,
@@ -268,9 +267,6 @@ class RegistrationBatch {
   private:
     std::vector<Registration *> regs_;
     cudaStream_t master_ = nullptr;
-    std::vector<cudaStream_t> branch_;
-    cudaEvent_t fork_ = nullptr;
-    std::vector<cudaEvent_t> join_;
     int *done_host_ = nullptr;  // page-locked copies of the pairs' done flags
     double last_ms_ = 0.0;
 };
@@ -300,7 +296,7 @@ class PriorTransform {
     int sweep_ = 0;
 };
 
-// default transform precision: BINDER_B200_PRECISION (0 FP32 SIMT, 1 3xTF32, 2 TF32) or 3xTF32
+// default transform precision: BINDER_B200_PRECISION (a TransformPrecision, 0 to 4) or the BF16 split
 int default_precision();
 // default tensor-core pass kind: BINDER_B200_PERSISTENT (0 per-tile CTAs, 1 persistent) or 0
 bool default_persistent();

@@ -224,11 +224,20 @@ void HartleyMatrix::init(int n_, cudaStream_t s) {
     cols = (n / 2 + 1 + 3) / 4 * 4;
     std::vector<double> host((size_t)2 * rows * cols, 0.0);
     const double pi = 3.14159265358979323846;
+    // n angles serve all the entries (a cosine and a sine per entry took 0.7 ms for the three
+    // axes of a 160 x 192 x 160 grid)
+    std::vector<double> ct(n), st(n);
+    for (int m = 0; m < n; ++m) {
+        const double ang = 2.0 * pi * (double)m / n;
+        ct[m] = std::cos(ang);
+        st[m] = std::sin(ang);
+    }
     for (int k = 0; k <= n / 2; ++k)
-        for (int j = 0; j <= n / 2; ++j) {
-            const double ang = 2.0 * pi * (double)(((long)j * k) % n) / n;
-            host[(size_t)k * cols + j] = std::cos(ang);
-            host[(size_t)(rows + k) * cols + j] = std::sin(ang);
+        for (int j = 0, m = 0; j <= n / 2; ++j) {
+            host[(size_t)k * cols + j] = ct[m];  // m = j k mod n
+            host[(size_t)(rows + k) * cols + j] = st[m];
+            m += k;
+            if (m >= n) m -= n;
         }
     dev = dev_alloc_n<double>(host.size(), s);
     BINDER_CUDA(cudaMemcpyAsync(dev, host.data(), host.size() * sizeof(double),

@@ -81,9 +81,8 @@ struct DBuf {
 
 void dct_upsample_matrix(int n, int m, std::vector<double> &U) {
     BINDER_CHECK(n >= 1 && m >= n, "spectral up-sampling needs an output axis at least as long");
-    std::vector<double> Cn((size_t)n * n), Cm((size_t)m * m);
-    dct2_matrix(n, Cn.data());  // Cn[k*n + j]: basis k at sample j
-    dct2_matrix(m, Cm.data());
+    const std::vector<double> &Cn = dct2_matrix(n);  // Cn[k*n + j]: basis k at sample j
+    const std::vector<double> &Cm = dct2_matrix(m);
     U.assign((size_t)m * n, 0.0);
     for (int jo = 0; jo < m; ++jo)
         for (int j = 0; j < n; ++j) {

@@ -272,9 +272,9 @@ void launch_axis_pass(const AxisArgs<T> &a, int mode, int ncomp, cudaStream_t st
 
 template void launch_axis_pass<float>(const AxisArgs<float> &, int, int, cudaStream_t);
 
-void dct2_matrix(int n, double *out) {
+const std::vector<double> &dct2_matrix(int n) {
     // each size is built once per process (n^2 cosines: about 1.4 ms for the three axes of a
-    // 160 x 192 x 160 grid, paid by every new registration otherwise) and copied from then on
+    // 160 x 192 x 160 grid, paid by every new registration otherwise) and stays as it is from then on
     static std::mutex mu;
     static std::map<int, std::vector<double>> built;
     std::lock_guard<std::mutex> lock(mu);
@@ -290,7 +290,7 @@ void dct2_matrix(int n, double *out) {
             }
         }
     }
-    std::copy(C.begin(), C.end(), out);
+    return C;
 }
 
 namespace {

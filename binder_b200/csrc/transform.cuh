@@ -7,6 +7,8 @@
 // n x 64 slab in shared memory and runs a register-blocked SIMT product over it.
 #pragma once
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace binder {
@@ -84,7 +86,8 @@ void launch_prior_noise(float *noise, long V, int ncomp, int chain_comps, uint64
 template <typename T>
 void launch_axis_pass(const AxisArgs<T> &a, int mode, int ncomp, cudaStream_t stream);
 
-// host-built orthonormal DCT-II matrix (rows = frequency) in double precision
-void dct2_matrix(int n, double *out);
+// host-built orthonormal DCT-II matrix [n][n] (rows = frequency) in double precision, built once
+// per size and never changed, so the reference stays good for the process
+const std::vector<double> &dct2_matrix(int n);
 
 }  // namespace binder

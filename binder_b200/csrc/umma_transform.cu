@@ -1279,32 +1279,57 @@ void launch_pt(const UArgs &a, cudaStream_t s) {
     else launch_pt_s<MODE, PLANES, 2>(a, pt_smem<MODE, PLANES, 2>(a.Npad), s);
 }
 
-float tf32_rna_host(float x) {
-    uint32_t u;
-    std::memcpy(&u, &x, 4);
+// FP32 -> TF32, round to nearest with ties away from zero
+__device__ __forceinline__ float tf32_rna(float x) {
+    uint32_t u = __float_as_uint(x);
     if ((u & 0x7f800000u) != 0x7f800000u) {
         u += 0x1000u;
         u &= 0xFFFFE000u;
     }
-    float r;
-    std::memcpy(&r, &u, 4);
-    return r;
+    return __uint_as_float(u);
 }
 
-// FP32 -> BF16 bits, round to nearest even (NaN kept a quiet NaN); host side of the B planes
-uint16_t bf16_rne_host(float x) {
-    uint32_t u;
-    std::memcpy(&u, &x, 4);
+// FP32 -> BF16 bits, round to nearest even (NaN kept a quiet NaN)
+__device__ __forceinline__ uint16_t bf16_rne(float x) {
+    uint32_t u = __float_as_uint(x);
     if ((u & 0x7f800000u) == 0x7f800000u) return (uint16_t)((u >> 16) | ((u & 0xffffu) ? 0x40u : 0u));
     u += 0x7fffu + ((u >> 16) & 1u);
     return (uint16_t)(u >> 16);
 }
 
-float bf16_to_float_host(uint16_t b) {
-    const uint32_t u = (uint32_t)b << 16;
-    float f;
-    std::memcpy(&f, &u, 4);
-    return f;
+// The operand planes of an n x n matrix M and of its transpose, and the transpose itself, from M:
+// one thread per element (k, j) of the padded planes, blockIdx.y = 1 for the transpose.  A few
+// hundred KB per axis, bound by its launch; formatted on the host, the same planes took most of
+// an object's set-up time (0.2 ms per axis of 160, and two copies and a wait each).
+__global__ void format_matrix_kernel(const float *M, float *MT, UmmaMatrix fwd, UmmaMatrix inv) {
+    const bool tr = blockIdx.y == 1;
+    const UmmaMatrix &U = tr ? inv : fwd;
+    const int n = U.n;
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = f % (U.nkc * kKC), k = f / (U.nkc * kKC);
+    if (k >= U.Npad) return;
+    const bool in = j < n && k < n;
+    const float v = !in ? 0.0f : tr ? M[(size_t)j * n + k] : M[(size_t)k * n + j];
+    if (tr && in) MT[(size_t)k * n + j] = v;
+    const size_t plane = (size_t)U.Npad * kKC;
+    const int kc = j / kKC, jj = j % kKC;
+    {
+        const float hi = tf32_rna(v), lo = tf32_rna(v - hi);
+        float *p = U.dev + (size_t)kc * 2 * plane + (size_t)(jj / 4) * (U.Npad * 4) +
+                   (k / 8) * 32 + (k % 8) * 4 + (jj % 4);
+        p[0] = hi;
+        p[plane] = lo;
+    }
+    {
+        // the same chunks as BF16 (2-byte elements, the same canonical layout: 16-byte K columns
+        // of 8 elements Npad * 16 bytes apart, 8-row groups 128 bytes apart)
+        const uint16_t hi = bf16_rne(v);
+        const uint16_t lo = bf16_rne(v - __uint_as_float((uint32_t)hi << 16));
+        uint16_t *p = U.dev16 + (size_t)kc * 2 * plane + (size_t)(jj / 8) * (U.Npad * 8) +
+                      (k / 8) * 64 + (k % 8) * 8 + (jj % 8);
+        p[0] = hi;
+        p[plane] = lo;
+    }
 }
 
 template <int MODE, int PLANES>
@@ -1339,51 +1364,24 @@ void launch_umma(const UArgs &a, int ncomp, cudaStream_t s) {
 }  // namespace
 
 // ------------------------------------------------------------------------------------------
-void UmmaMatrix::init(const double *M, int n_, cudaStream_t s) {
+size_t UmmaMatrix::elements(int n) {
+    return (size_t)((n + kKC - 1) / kKC) * 2 * (size_t)(((n + 15) / 16) * 16) * kKC;
+}
+
+void UmmaMatrix::attach(int n_, float *planes, uint16_t *planes16) {
     n = n_;
     Npad = ((n + 15) / 16) * 16;
     nkc = (n + kKC - 1) / kKC;
-    const size_t plane = (size_t)Npad * kKC;
-    std::vector<float> host((size_t)nkc * 2 * plane, 0.0f);
-    for (int kc = 0; kc < nkc; ++kc)
-        for (int k = 0; k < n; ++k)
-            for (int jj = 0; jj < kKC; ++jj) {
-                const int j = kc * kKC + jj;
-                if (j >= n) continue;
-                const float v = (float)M[(size_t)k * n + j];
-                const float hi = tf32_rna_host(v);
-                const float lo = tf32_rna_host(v - hi);
-                const size_t off = (size_t)(jj / 4) * (Npad * 4) + (k / 8) * 32 + (k % 8) * 4 + (jj % 4);
-                host[(size_t)kc * 2 * plane + off] = hi;
-                host[(size_t)kc * 2 * plane + plane + off] = lo;
-            }
-    // the same chunks as BF16 hi / lo planes (2-byte elements, the same canonical layout: 16-byte
-    // K columns of 8 elements Npad * 16 bytes apart, 8-row groups 128 bytes apart)
-    std::vector<uint16_t> host16((size_t)nkc * 2 * plane, 0);
-    for (int kc = 0; kc < nkc; ++kc)
-        for (int k = 0; k < n; ++k)
-            for (int jj = 0; jj < kKC; ++jj) {
-                const int j = kc * kKC + jj;
-                if (j >= n) continue;
-                const float v = (float)M[(size_t)k * n + j];
-                const uint16_t hi = bf16_rne_host(v);
-                const uint16_t lo = bf16_rne_host(v - bf16_to_float_host(hi));
-                const size_t off = (size_t)(jj / 8) * (Npad * 8) + (k / 8) * 64 + (k % 8) * 8 + (jj % 8);
-                host16[(size_t)kc * 2 * plane + off] = hi;
-                host16[(size_t)kc * 2 * plane + plane + off] = lo;
-            }
-    dev = dev_alloc_n<float>(host.size(), s);
-    dev16 = dev_alloc_n<uint16_t>(host16.size(), s);
-    BINDER_CUDA(cudaMemcpyAsync(dev, host.data(), host.size() * sizeof(float),
-                                cudaMemcpyHostToDevice, s));
-    BINDER_CUDA(cudaMemcpyAsync(dev16, host16.data(), host16.size() * sizeof(uint16_t),
-                                cudaMemcpyHostToDevice, s));
-    BINDER_CUDA(cudaStreamSynchronize(s));  // `host` goes out of scope
+    dev = planes;
+    dev16 = planes16;
 }
 
-void UmmaMatrix::release(cudaStream_t s) {
-    dev_free_p(dev, s);
-    dev_free_p(dev16, s);
+void launch_format_matrix(const float *M, float *MT, const UmmaMatrix &fwd, const UmmaMatrix &inv,
+                          cudaStream_t s) {
+    const int count = fwd.nkc * kKC * fwd.Npad;
+    count_launch(), format_matrix_kernel<<<dim3((count + 255) / 256, 2), 256, 0, s>>>(M, MT, fwd,
+                                                                                      inv);
+    BINDER_CUDA(cudaGetLastError());
 }
 
 void launch_axis_pass_tc(const AxisArgs<float> &b, const UmmaMatrix &M1, const UmmaMatrix *M2,

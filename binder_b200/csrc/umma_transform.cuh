@@ -12,10 +12,15 @@ struct UmmaMatrix {
     int n = 0, Npad = 0, nkc = 0;
     float *dev = nullptr;
     uint16_t *dev16 = nullptr;  // the same chunks as BF16 hi / lo planes (2-byte elements)
-    // device copy from the stream-ordered pool on stream s (synchronised before returning)
-    void init(const double *M, int n, cudaStream_t s);
-    void release(cudaStream_t s);
+    // elements of dev and of dev16 (the padding included) for an n x n matrix
+    static size_t elements(int n);
+    // take the caller's device buffers of elements(n) each
+    void attach(int n, float *planes, uint16_t *planes16);
 };
+
+// write MT = M^T and the planes of M (fwd) and M^T (inv) on stream s; M [n][n] on the device
+void launch_format_matrix(const float *M, float *MT, const UmmaMatrix &fwd, const UmmaMatrix &inv,
+                          cudaStream_t s);
 
 // precision of the DCT passes
 enum TransformPrecision : int {
