@@ -213,6 +213,7 @@ void MStep::init(int x, int y, int z, cudaStream_t s, int nchains) {
         const char *e = std::getenv("BINDER_B200_FUSED2D");
         const bool off = e && e[0] == '0' && e[1] == 0;
         fused2d = chains == 1 && !off && z == 1 && x <= kM2dMaxN && y <= kM2dMaxN;
+        if (fused2d) fused_cluster = mstep2d_cluster(e && e[0] == '8' && e[1] == 0);
     }
 }
 
@@ -283,7 +284,8 @@ void MStep::enqueue(const float *r, float *d, const float *xpos, const float *D,
         a.D = D; a.sigma2 = sigma2; a.sample = sample; a.want_raw = want_raw;
         a.every = every < 1 ? 1 : every; a.seed = seed; a.chain = chain; a.rho_p = rho_p;
         for (int n = 0; n < 3; ++n) a.eta2[n] = eta2[n];
-        launch_mstep2d(a, r, d, nx, ny, dct.fwd[0], dct.inv[0], dct.fwd[1], dct.inv[1], s);
+        launch_mstep2d(a, r, d, nx, ny, dct.fwd[0], dct.inv[0], dct.fwd[1], dct.inv[1],
+                       fused_cluster, s);
         return;
     }
     a.D = D; a.sigma2 = sigma2; a.sample = sample; a.want_raw = want_raw;

@@ -34,6 +34,7 @@ struct MStep {
     bool persistent = false;
     // 2D images up to 128 x 128: the whole M-step in one launch (mstep2d.cu)
     bool fused2d = false;
+    int fused_cluster = 8;  // its CTAs per component
     // the tensor-core passes of components 1 and 2 run on their own streams (graph branches), so
     // one component's last partial wave of tiles overlaps the other components' passes
     cudaStream_t side[2] = {nullptr, nullptr};
