@@ -6,6 +6,7 @@
 // reference CPU backend's bit for bit on the same FP64 input.
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "layout.cuh"
@@ -39,7 +40,6 @@ struct Red {
     unsigned long long mn, mx;
     unsigned long long below, above, negative;
     double sum[3];
-    int count;  // flagged cells (limiter list length)
     int pad;
 };
 
@@ -240,13 +240,6 @@ __global__ void gradient_kernel(const double *pos, int nx, int ny, int nz, doubl
     }
 }
 
-// the limiter step of one flagged corner (topology_correction_3D.cpp:279-345,
-// topology_correction_2D.cpp:257-309): J the corner's N x N gradient matrix (column n2 read at
-// vertex n2), replaced by (1 - a) J + a I.  The reference steps
-// alpha by 0.1 (capped at 1) until det((1 - alpha) J + alpha I) lies in [e1, e2], at most 11
-// steps, then takes one step more.  The alphas are constants, so the trial determinants are
-// evaluated independently, a group at a time (the same expressions the loop evaluates), and the
-// first one in range picks the step: the walk, one corner after another, gains the ILP.
 template <int N>
 __device__ __forceinline__ double detn(const double (&J)[N][N]) {
     if constexpr (N == 2)
@@ -255,272 +248,234 @@ __device__ __forceinline__ double detn(const double (&J)[N][N]) {
         return det3(J[0][0], J[0][1], J[0][2], J[1][0], J[1][1], J[1][2], J[2][0], J[2][1], J[2][2]);
 }
 
-template <int N>
-__device__ __forceinline__ void limit_corner(double (&J)[N][N], double e1, double e2,
-                                             bool &capped) {
-    constexpr int kSteps = 11;
-    double al[kSteps + 2];  // al[k]: alpha after k steps (constant-folded)
-    al[0] = 0.0;
-#pragma unroll
-    for (int k = 1; k < kSteps + 2; ++k) {
-        al[k] = al[k - 1] + 0.1;
-        if (al[k] > 1.0) al[k] = 1.0;
-    }
-    const double det0 = detn<N>(J);
-    // k steps taken (the first k whose determinant lies in [e1, e2]): the final alpha is al[k + 1]
-    double alpha = al[1];
-    if (det0 > e2 || det0 < e1) {
-        bool none = true;  // alpha == 1 (identity) tried as well: [e1, e2] misses 1
-        alpha = al[kSteps + 1];
-        // trials in groups of kGroup (independent within a group), stopping at the first group
-        // with a determinant in range
-        constexpr int kGroup = 4;
-#pragma unroll
-        for (int t0 = 1; t0 <= kSteps; t0 += kGroup) {
-            const int t1 = t0 + kGroup - 1 < kSteps ? t0 + kGroup - 1 : kSteps;
-#pragma unroll
-            for (int t = t1; t >= t0; --t) {
-                const double a = al[t];
-                double Jn[N][N];
-                for (int n1 = 0; n1 < N; ++n1)
-                    for (int n2 = 0; n2 < N; ++n2)
-                        Jn[n1][n2] = (1 - a) * J[n1][n2] + a * (n1 == n2 ? 1.0 : 0.0);
-                const double det = detn<N>(Jn);
-                if (!(det > e2 || det < e1)) {
-                    alpha = al[t + 1];
-                    none = false;
-                }
-            }
-            if (!none) break;
-        }
-        if (none) capped = true;
-    }
-    for (int n1 = 0; n1 < N; ++n1)
-        for (int n2 = 0; n2 < N; ++n2)
-            J[n1][n2] = (1 - alpha) * J[n1][n2] + alpha * (n1 == n2 ? 1.0 : 0.0);
-}
-
-// limit_corner by a group of 16 lanes holding the same J: lane t (1 <= t <= 11) evaluates trial
-// t, and the lowest lane whose determinant lies in [e1, e2] picks the step.  The same expressions
-// and the same choice as limit_corner; every lane of the group ends with the new J.  gmask names
-// the group's lanes, which all take this call together.
-__device__ __forceinline__ void limit_corner_lanes(double (&J)[2][2], double e1, double e2,
-                                                   bool &capped, int gl, unsigned gmask,
-                                                   double at, double an) {
-    const double det0 = J[0][0] * J[1][1] - J[0][1] * J[1][0];
-    double alpha = 0.1;  // one step from 0
-    if (det0 > e2 || det0 < e1) {  // uniform across the group
-        bool in = false;
-        if (gl >= 1 && gl <= 11) {
-            double Jn[2][2];
-            for (int n1 = 0; n1 < 2; ++n1)
-                for (int n2 = 0; n2 < 2; ++n2)
-                    Jn[n1][n2] = (1 - at) * J[n1][n2] + at * (n1 == n2 ? 1.0 : 0.0);
-            const double det = Jn[0][0] * Jn[1][1] - Jn[0][1] * Jn[1][0];
-            in = !(det > e2 || det < e1);
-        }
-        const unsigned b = __ballot_sync(gmask, in) & gmask;
-        const int k = b ? __ffs((int)b) - 1 : -1;  // lane of the warp
-        alpha = __shfl_sync(gmask, an, k < 0 ? 11 : (k & 15), 16);  // al[k + 1], or al[12] = 1
-        if (k < 0) capped = true;
-    }
-    for (int n1 = 0; n1 < 2; ++n1)
-        for (int n2 = 0; n2 < 2; ++n2)
-            J[n1][n2] = (1 - alpha) * J[n1][n2] + alpha * (n1 == n2 ? 1.0 : 0.0);
-}
-
-// topology_correction_3D.cpp:247-332.  The reference visits cells in lexicographic order and a
-// cell's 8 corners in order; a cell reads and writes gradients only inside its 2x2x2 footprint,
-// so two cells interact only if they differ by at most 1 along every axis.  A flagged cell may
-// therefore go as soon as its flagged neighbours that come before it have gone: cells with none go
-// first (round 0), and each cell counts down its later neighbours, the last count putting one into
-// the next round.  The cells of a round are no neighbours of each other, so the result is the
-// sequential walk's exactly, and the rounds are as many as the longest chain of neighbouring cells:
-// 42 for a 160x192x160 field with 157,751 flagged cells, where a wavefront over the whole volume
-// (4x + 2y + z, one CTA) has 1,157 levels and took 3.1 ms; the rounds take 0.2 ms.
+// topology_correction_3D.cpp:247-332 and topology_correction_2D.cpp:248-313.  The reference visits
+// cells in lexicographic order and a cell's corners in order; a cell reads and writes gradients only
+// inside its 2x2x2 (2x2) footprint, so two cells interact only if they differ by at most 1 along
+// every axis.  A flagged cell may therefore go as soon as its flagged neighbours that come before it
+// have gone: cells with none go first (round 0), and each cell counts down its later neighbours, the
+// last count putting one into the next round.  The cells of a round are no neighbours of each other,
+// so the result is the sequential walk's exactly, and the rounds are as many as the longest chain of
+// neighbouring cells: 42 for a 160x192x160 field with 157,751 flagged cells, 58 for a 128x128 one
+// with 2,253.
+//
+// A step: J is a corner's matrix of gradients, replaced by (1 - alpha) J + alpha I.  The reference
+// steps alpha by 0.1 (capped at 1) until det((1 - alpha) J + alpha I) lies in [e1, e2], at most 11
+// steps from 0, then takes one step more.  The alphas are constants, so the trials are independent:
+// four lanes share a cell and try four alphas at a time, and the lowest trial in range picks the
+// step.  The field's values of a cell stay in shared memory from its first corner to its last.
+// FP64 work and the chain of a cell's corners bound it: with 16 lanes to a cell, all twelve trials
+// at once and the values passed around by shuffles, one CTA took 153 us where this takes 138
+// (22x24x24, 6,517 flagged cells, 130 rounds); a wavefront over the levels 2x + y of an image took
+// 130 us where the rounds take 38 (128x128).
 struct LimiterArgs {
-    const uint8_t *mask;  // flagged corners of every cell (corner_kernel)
-    double *g;            // gradients [9][V]
+    const uint8_t *mask;  // flagged corners of every cell (corner_kernel, corner2d_kernel)
+    double *g;            // gradients [N * N][V]
     int *deg;             // earlier flagged neighbours still to go, per cell
     int *front[2];        // the cells of a round and of the next
     int *counts;          // cells of each round
-    int nx, ny, nz;
+    int nx, ny, nz;       // nz = 1: an image
     double e1, e2;
     unsigned *flags;
 };
 
-// neighbour q (0 .. 12) of the 13 that come later in lexicographic order: (dx, dy, dz) > 0
-__device__ __forceinline__ void later_neighbour(int q, int &dx, int &dy, int &dz) {
-    const int o = q + 14;  // 27 offsets in order, the cell itself is the 14th
-    dx = o / 9 - 1;
-    dy = o / 3 % 3 - 1;
-    dz = o % 3 - 1;
+constexpr int kTrials = 12;  // alphas of 0 .. 11 steps
+// al[k]: alpha after k steps, k <= kTrials
+__device__ __forceinline__ void step_alphas(double *al) {
+    double a = 0.0;
+    for (int k = 0; k <= kTrials; ++k) {
+        al[k] = a;
+        a = a + 0.1;
+        if (a > 1.0) a = 1.0;
+    }
 }
 
-// The corners of one cell by a group of 16 lanes (gmask).  The 36 gradient entries its corners read
-// -- column n2 at the four vertices with coordinate n2 zero -- are loaded at once, entry i by lane
-// i % 16, and stay in the lanes until the end.  Per corner every lane gathers the 3x3 matrix; lane
-// t evaluates trial t of the limiter step (1 <= t <= 11, alpha `at`, the alpha after one step more
-// `an`), and the lowest lane whose determinant lies in [e1, e2] picks the step: limit_corner's
-// expressions and choice.
+// a grid of cells: how a flat index, the later neighbours and a cell's values are laid out
+template <int DIM>
+struct CellGrid {
+    static constexpr int kLater = DIM == 3 ? 13 : 4;    // later neighbours in lexicographic order
+    static constexpr int kPerLane = DIM == 3 ? 9 : 2;   // of the 36 (8) values, by 4 lanes
+    static constexpr int kStride = 4 * kPerLane + 1;    // doubles of scratch per cell
+    int cx, cy, cz;
+    __device__ __forceinline__ explicit CellGrid(const LimiterArgs &a)
+        : cx(a.nx - 1), cy(a.ny - 1), cz(DIM == 3 ? a.nz - 1 : 1) {}
+    __device__ __forceinline__ int count() const { return cx * cy * cz; }
+    __device__ __forceinline__ void at(int cell, int &x, int &y, int &z) const {
+        const int row = DIM == 3 ? cell / cz : cell;
+        z = DIM == 3 ? cell - row * cz : 0;
+        x = row / cy;
+        y = row - x * cy;
+    }
+    // the later neighbour q of (x, y, z), or the earlier one with sign -1; -1 outside
+    __device__ __forceinline__ int neighbour(int q, int sign, int x, int y, int z) const {
+        const int o = q + kLater + 1;  // 27 (9) offsets in order, the cell itself in the middle
+        const int X = x + sign * (DIM == 3 ? o / 9 - 1 : o / 3 - 1);
+        const int Y = y + sign * (DIM == 3 ? o / 3 % 3 - 1 : o % 3 - 1);
+        const int Z = DIM == 3 ? z + sign * (o % 3 - 1) : 0;
+        const bool in = (unsigned)X < (unsigned)cx && (unsigned)Y < (unsigned)cy &&
+                        (DIM == 2 || (unsigned)Z < (unsigned)cz);
+        return in ? (X * cy + Y) * cz + Z : -1;
+    }
+    // earlier flagged neighbours of a flagged cell
+    __device__ __forceinline__ int earlier_flagged(const uint8_t *mask, int cell) const {
+        int x, y, z, n = 0;
+        at(cell, x, y, z);
+#pragma unroll
+        for (int q = 0; q < kLater; ++q) {
+            const int nb = neighbour(q, -1, x, y, z);
+            if (nb >= 0) n += mask[nb] != 0;
+        }
+        return n;
+    }
+};
+
+// The flagged corners (`mask`) of one cell by four lanes (gl = 0 .. 3, gmask).  Column n2 of a
+// corner's matrix is read at the corner's vertex with its n2 bit cleared, so the values are
+// s[(n2 N + n1) 4 + p] (3D: p the two other bits of the vertex) and s[n2 4 + n1 2 + p] (2D: p the
+// other bit); lane gl loads and stores s[4 e + gl].
+template <int DIM>
 __device__ __forceinline__ void limit_cell(const LimiterArgs &a, int x, int y, int z, unsigned mask,
-                                           int gl, unsigned gmask, double at, double an,
+                                           int gl, unsigned gmask, double *s, const double *al,
                                            bool &capped) {
+    constexpr int E = CellGrid<DIM>::kPerLane;
     const long V = (long)a.nx * a.ny * a.nz;
-    double v[3];
-    double *src[3];
+    double *src[DIM];  // of entry (n1, n2): src[n2] + n1 * DIM * V
+    if constexpr (DIM == 3) {
+        const int p = gl >> 1, q = gl & 1;
+        src[0] = a.g + ((long)x * a.ny + (y + p)) * a.nz + (z + q);
+        src[1] = a.g + V + ((long)(x + p) * a.ny + y) * a.nz + (z + q);
+        src[2] = a.g + 2 * V + ((long)(x + p) * a.ny + (y + q)) * a.nz + z;
+    } else {
+        const int n1 = gl >> 1, p = gl & 1;
+        src[0] = a.g + (n1 * 2) * V + (long)x * a.ny + (y + p);
+        src[1] = a.g + (n1 * 2 + 1) * V + (long)(x + p) * a.ny + y;
+    }
+    double v[E];
 #pragma unroll
-    for (int e = 0; e < 3; ++e) {
-        const int i = gl + 16 * e;
-        if (i < 36) {
-            const int n2 = i / 12, n1 = i / 4 % 3, p = (i >> 1) & 1, q = i & 1;
-            const int ox = n2 == 0 ? 0 : p, oy = n2 == 0 ? p : (n2 == 1 ? 0 : q),
-                      oz = n2 == 2 ? 0 : q;
-            src[e] = a.g + (n1 * 3 + n2) * V + ((long)(x + ox) * a.ny + (y + oy)) * a.nz + (z + oz);
-            v[e] = *src[e];
-        } else {
-            src[e] = nullptr;
-            v[e] = 0.0;
+    for (int e = 0; e < E; ++e) v[e] = DIM == 3 ? src[e / 3][(e % 3) * 3 * V] : *src[e % DIM];
+#pragma unroll
+    for (int e = 0; e < E; ++e) s[4 * e + gl] = v[e];
+    __syncwarp(gmask);
+    for (; mask; mask &= mask - 1) {
+        const int c = __ffs((int)mask) - 1;
+        // the corner's vertex: 000, 100, 010, 001, 011, 101, 110, 111, or 00, 10, 01, 11
+        const int va = DIM == 3 ? 0xE2 >> c & 1 : c & 1, vb = DIM == 3 ? 0xD4 >> c & 1 : c >> 1,
+                  vc = 0xB8 >> c & 1;
+        const int col[3] = {DIM == 3 ? vb * 2 + vc : vb, DIM == 3 ? 12 + va * 2 + vc : 4 + va,
+                            24 + va * 2 + vb};
+        constexpr int kRow = DIM == 3 ? 4 : 2;
+        double J[DIM][DIM];
+#pragma unroll
+        for (int n1 = 0; n1 < DIM; ++n1)
+#pragma unroll
+            for (int n2 = 0; n2 < DIM; ++n2) J[n1][n2] = s[col[n2] + n1 * kRow];
+        // the entries this lane replaces: e = n2 DIM + n1 = gl, gl + 4, gl + 8
+        constexpr int kOwn = DIM == 3 ? 3 : 1;
+        double own[kOwn];
+        int at[kOwn];
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i) {
+            const int e = gl + 4 * i, n2 = e / DIM, n1 = e - n2 * DIM;
+            at[i] = (n2 == 0 ? col[0] : n2 == 1 ? col[1] : col[2]) + n1 * kRow;
+            own[i] = e < DIM * DIM ? s[at[i]] : 0.0;
         }
-    }
-    constexpr int vert[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1},
-                                {0, 1, 1}, {1, 0, 1}, {1, 1, 0}, {1, 1, 1}};
+        // trial t: alpha after t steps; the lowest trial whose determinant is in range takes one
+        // step more (trial 0 is J itself)
+        int t = -1;
+#pragma unroll 1
+        for (int b = 0; b < kTrials && t < 0; b += 4) {
+            const double at1 = al[b + gl];
+            double Jn[DIM][DIM];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        if (!(mask >> c & 1u)) continue;  // uniform across the group
-        const int va = vert[c][0], vb = vert[c][1], vc = vert[c][2];
-        const int at0[3] = {vb * 2 + vc, va * 2 + vc, va * 2 + vb};
-        double J[3][3];
+            for (int n1 = 0; n1 < DIM; ++n1)
 #pragma unroll
-        for (int n1 = 0; n1 < 3; ++n1)
-#pragma unroll
-            for (int n2 = 0; n2 < 3; ++n2) {
-                const int i = (n2 * 3 + n1) * 4 + at0[n2];
-                J[n1][n2] = __shfl_sync(gmask, v[i >> 4], i & 15, 16);
-            }
-        const double det0 = detn<3>(J);
-        double alpha = 0.1;  // one step from 0
-        if (det0 > a.e2 || det0 < a.e1) {
-            bool in = false;
-            if (gl >= 1 && gl <= 11) {
-                double Jn[3][3];
-#pragma unroll
-                for (int n1 = 0; n1 < 3; ++n1)
-#pragma unroll
-                    for (int n2 = 0; n2 < 3; ++n2)
-                        Jn[n1][n2] = (1 - at) * J[n1][n2] + at * (n1 == n2 ? 1.0 : 0.0);
-                const double det = detn<3>(Jn);
-                in = !(det > a.e2 || det < a.e1);
-            }
-            const unsigned b = __ballot_sync(gmask, in) & gmask;
-            const int k = b ? __ffs((int)b) - 1 : -1;  // lane of the warp
-            alpha = __shfl_sync(gmask, an, k < 0 ? 11 : (k & 15), 16);  // al[k + 1], or al[12] = 1
-            if (k < 0) capped = true;
+                for (int n2 = 0; n2 < DIM; ++n2)
+                    Jn[n1][n2] = (1 - at1) * J[n1][n2] + at1 * (n1 == n2 ? 1.0 : 0.0);
+            const double det = detn<DIM>(Jn);
+            const unsigned in = __ballot_sync(gmask, !(det > a.e2 || det < a.e1)) & gmask;
+            if (in) t = b + ((__ffs((int)in) - 1) & 3);
         }
+        if (t < 0) capped = true;
+        const double alpha = al[t < 0 ? kTrials : t + 1];
 #pragma unroll
-        for (int n1 = 0; n1 < 3; ++n1)
-#pragma unroll
-            for (int n2 = 0; n2 < 3; ++n2) {
-                const int i = (n2 * 3 + n1) * 4 + at0[n2];
-                const double w = (1 - alpha) * J[n1][n2] + alpha * (n1 == n2 ? 1.0 : 0.0);
-                if (gl == (i & 15)) v[i >> 4] = w;
-            }
+        for (int i = 0; i < kOwn; ++i) {
+            const int e = gl + 4 * i, n2 = e / DIM, n1 = e - n2 * DIM;
+            if (e < DIM * DIM)
+                s[at[i]] = (1 - alpha) * own[i] + alpha * (n1 == n2 ? 1.0 : 0.0);
+        }
+        __syncwarp(gmask);
     }
 #pragma unroll
-    for (int e = 0; e < 3; ++e)
-        if (src[e]) *src[e] = v[e];
-}
-
-// the limiter's alphas after t steps and after t + 1 (0.1 at a time, capped at 1)
-__device__ __forceinline__ void trial_alphas(int t, double &at, double &an) {
-    at = 0.0;
-    for (int k = 0; k < t; ++k) {
-        at = at + 0.1;
-        if (at > 1.0) at = 1.0;
-    }
-    an = at + 0.1;
-    if (an > 1.0) an = 1.0;
-}
-
-// earlier flagged neighbours of a flagged cell
-__device__ __forceinline__ int earlier_flagged(const uint8_t *mask, int x, int y, int z, int cx,
-                                               int cy, int cz) {
-    int n = 0;
-#pragma unroll
-    for (int q = 0; q < 13; ++q) {
-        int dx, dy, dz;
-        later_neighbour(q, dx, dy, dz);
-        const int X = x - dx, Y = y - dy, Z = z - dz;
-        if (X >= 0 && Y >= 0 && Z >= 0 && X < cx && Y < cy && Z < cz)
-            n += mask[((long)X * cy + Y) * cz + Z] != 0;
-    }
-    return n;
+    for (int e = 0; e < E; ++e)
+        (DIM == 3 ? src[e / 3][(e % 3) * 3 * V] : *src[e % DIM]) = s[4 * e + gl];
+    __syncwarp(gmask);  // the scratch is free for the group's next cell
 }
 
 // round 0: the flagged cells with no earlier flagged neighbour
 __global__ void limiter_start_kernel(const LimiterArgs a) {
-    const int cx = a.nx - 1, cy = a.ny - 1, cz = a.nz - 1;
-    const long cells = (long)cx * cy * cz;
-    for (long cell = (long)blockIdx.x * blockDim.x + threadIdx.x; cell < cells;
-         cell += (long)gridDim.x * blockDim.x) {
+    const CellGrid<3> grid(a);
+    const int cells = grid.count();
+    for (int cell = blockIdx.x * blockDim.x + threadIdx.x; cell < cells;
+         cell += gridDim.x * blockDim.x) {
         if (!a.mask[cell]) continue;
-        const int x = (int)(cell / ((long)cy * cz)), y = (int)((cell / cz) % cy),
-                  z = (int)(cell % cz);
-        const int n = earlier_flagged(a.mask, x, y, z, cx, cy, cz);
+        const int n = grid.earlier_flagged(a.mask, cell);
         a.deg[cell] = n;
-        if (n == 0) a.front[0][atomicAdd(&a.counts[0], 1)] = (int)cell;
+        if (n == 0) a.front[0][atomicAdd(&a.counts[0], 1)] = cell;
     }
 }
 
 // one round over the whole GPU
-__global__ void __launch_bounds__(256) limiter_round_kernel(const LimiterArgs a, int round) {
+constexpr int kRoundThreads = 256;
+__global__ void __launch_bounds__(kRoundThreads) limiter_round_kernel(const LimiterArgs a,
+                                                                      int round) {
+    __shared__ double al[kTrials + 1];
+    __shared__ double scratch[kRoundThreads / 4 * CellGrid<3>::kStride];
     const int n = a.counts[round];
-    const int gl = threadIdx.x & 15;
-    const unsigned gmask = 0xffffu << (threadIdx.x & 16);
-    const int cx = a.nx - 1, cy = a.ny - 1, cz = a.nz - 1;
-    const int *now = a.front[round & 1];
-    int *next = a.front[(round + 1) & 1];
-    double at, an;
-    trial_alphas(gl, at, an);
+    if (blockIdx.x * (kRoundThreads / 4) >= n) return;
+    if (threadIdx.x == 0) step_alphas(al);
+    __syncthreads();
+    const int gl = threadIdx.x & 3;
+    const unsigned gmask = 0xfu << (threadIdx.x & 28);
+    double *s = scratch + (threadIdx.x >> 2) * CellGrid<3>::kStride;
+    const CellGrid<3> grid(a);
+    const int *now = round & 1 ? a.front[1] : a.front[0];
+    int *next = round & 1 ? a.front[0] : a.front[1];
     bool capped = false;
-    for (int q = (blockIdx.x * 256 + threadIdx.x) >> 4; q < n; q += gridDim.x * 16) {
-        const long cell = now[q];
-        const int x = (int)(cell / ((long)cy * cz)), y = (int)((cell / cz) % cy),
-                  z = (int)(cell % cz);
-        limit_cell(a, x, y, z, a.mask[cell], gl, gmask, at, an, capped);
-        if (gl < 13) {
-            int dx, dy, dz;
-            later_neighbour(gl, dx, dy, dz);
-            const int X = x + dx, Y = y + dy, Z = z + dz;
-            if (X < cx && Y >= 0 && Y < cy && Z >= 0 && Z < cz) {
-                const long nb = ((long)X * cy + Y) * cz + Z;
-                if (a.mask[nb] && atomicSub(&a.deg[nb], 1) == 1)
-                    next[atomicAdd(&a.counts[round + 1], 1)] = (int)nb;
-            }
+    for (int q = (blockIdx.x * kRoundThreads + threadIdx.x) >> 2; q < n;
+         q += gridDim.x * (kRoundThreads / 4)) {
+        const int cell = now[q];
+        int x, y, z;
+        grid.at(cell, x, y, z);
+        limit_cell<3>(a, x, y, z, a.mask[cell], gl, gmask, s, al, capped);
+        for (int l = gl; l < CellGrid<3>::kLater; l += 4) {
+            const int nb = grid.neighbour(l, 1, x, y, z);
+            if (nb >= 0 && a.mask[nb] && atomicSub(&a.deg[nb], 1) == 1)
+                next[atomicAdd(&a.counts[round + 1], 1)] = nb;
         }
-        __syncwarp(gmask);
     }
     if (capped) atomicOr(a.flags, (unsigned)kFlagLimiterCapped);
 }
 
 // The rounds from `round` on, until none is left, in one CTA: small rounds cost less between two
-// barriers than as launches.  SM: a volume of at most kSmallCells cells, all rounds, with the masks,
-// counts and rounds in shared memory.
+// barriers than as launches.  SM: a grid of at most kSmallCells cells, all rounds, with the masks,
+// counts and rounds in shared memory.  `groups` of four lanes have scratch.
 constexpr int kSmallCells = 65536;
 constexpr int kTailThreads = 1024;
-template <bool SM>
+template <int DIM, bool SM>
 __global__ void __launch_bounds__(kTailThreads) limiter_tail_kernel(const LimiterArgs a, int round,
-                                                                    int cap) {
+                                                                    int cap, int groups) {
     extern __shared__ __align__(16) unsigned char shm[];
-    __shared__ int cnt[2];
-    const int cx = a.nx - 1, cy = a.ny - 1, cz = a.nz - 1;
-    const int cells = SM ? cx * cy * cz : 0, words = (cells + 3) >> 2;
-    unsigned *deg = reinterpret_cast<unsigned *>(shm);                       // [words] 4 counts each
-    uint8_t *mask = reinterpret_cast<uint8_t *>(deg + words);                // [4 * words]
+    __shared__ int cnt[3];  // of this round, the next, and the one after (cleared meanwhile)
+    __shared__ double al[kTrials + 1];
+    const CellGrid<DIM> grid(a);
+    const int cells = SM ? grid.count() : 0, words = (cells + 3) >> 2;
+    double *scratch = reinterpret_cast<double *>(shm);  // [groups][kStride]
+    unsigned *deg = reinterpret_cast<unsigned *>(scratch + (size_t)groups * grid.kStride);
+    uint8_t *mask = reinterpret_cast<uint8_t *>(deg + words);                    // deg: 4 to a word
     unsigned short *f16 = reinterpret_cast<unsigned short *>(mask + 4 * words);  // [2][cap]
-    const int tid = threadIdx.x, gl = tid & 15;
-    const unsigned gmask = 0xffffu << (tid & 16);
-    if (tid < 2) cnt[tid] = 0;
+    const int tid = threadIdx.x, gl = tid & 3;
+    const unsigned gmask = 0xfu << (tid & 28);
+    if (tid < 3) cnt[tid] = 0;
+    if (tid == 32) step_alphas(al);
     if (SM) {
         for (int i = tid; i < 4 * words; i += kTailThreads) mask[i] = i < cells ? a.mask[i] : 0;
         __syncthreads();
@@ -529,47 +484,45 @@ __global__ void __launch_bounds__(kTailThreads) limiter_tail_kernel(const Limite
             for (int e = 0; e < 4; ++e) {
                 const int cell = 4 * w + e;
                 if (cell >= cells || !mask[cell]) continue;
-                const int x = cell / (cy * cz), y = cell / cz % cy, z = cell % cz;
-                const unsigned n = (unsigned)earlier_flagged(mask, x, y, z, cx, cy, cz);
+                const unsigned n = (unsigned)grid.earlier_flagged(mask, cell);
                 d |= n << (8 * e);
                 if (n == 0) f16[atomicAdd(&cnt[0], 1)] = (unsigned short)cell;
             }
             deg[w] = d;
         }
     } else {
-        if (tid == 0) cnt[round & 1] = a.counts[round];
+        __syncthreads();
+        if (tid == 0) cnt[0] = a.counts[round];
     }
     __syncthreads();
-    double at, an;
-    trial_alphas(gl, at, an);
     bool capped = false;
-    for (;; ++round) {
-        const int cur = round & 1, n = cnt[cur];
-        if (n == 0) break;
-        for (int q = tid >> 4; q < n; q += kTailThreads / 16) {
-            const int cell = SM ? (int)f16[cur * cap + q] : a.front[cur][q];
-            const int x = cell / (cy * cz), y = cell / cz % cy, z = cell % cz;
-            limit_cell(a, x, y, z, SM ? mask[cell] : a.mask[cell], gl, gmask, at, an, capped);
-            if (gl < 13) {
-                int dx, dy, dz;
-                later_neighbour(gl, dx, dy, dz);
-                const int X = x + dx, Y = y + dy, Z = z + dz;
-                if (X < cx && Y >= 0 && Y < cy && Z >= 0 && Z < cz) {
-                    const int nb = (X * cy + Y) * cz + Z;
+    double *s = scratch + (size_t)(tid >> 2) * grid.kStride;
+    for (int r = 0;; ++r, ++round) {
+        const int n = cnt[r % 3], cur = round & 1;
+        if (n == 0) break;  // uniform: nothing writes this count until the next barrier
+        int *next = &cnt[(r + 1) % 3];
+        if (tid < 4 * groups)
+            for (int q = tid >> 2; q < n; q += groups) {
+                const int cell = SM ? (int)f16[cur * cap + q]
+                                    : (cur ? a.front[1] : a.front[0])[q];
+                int x, y, z;
+                grid.at(cell, x, y, z);
+                limit_cell<DIM>(a, x, y, z, SM ? mask[cell] : a.mask[cell], gl, gmask, s, al,
+                                capped);
+                for (int l = gl; l < grid.kLater; l += 4) {
+                    const int nb = grid.neighbour(l, 1, x, y, z);
+                    if (nb < 0) continue;
                     if (SM) {
                         const int sh = 8 * (nb & 3);
                         if (mask[nb] && (atomicSub(&deg[nb >> 2], 1u << sh) >> sh & 0xffu) == 1u)
-                            f16[(cur ^ 1) * cap + atomicAdd(&cnt[cur ^ 1], 1)] = (unsigned short)nb;
+                            f16[(cur ^ 1) * cap + atomicAdd(next, 1)] = (unsigned short)nb;
                     } else if (a.mask[nb] && atomicSub(&a.deg[nb], 1) == 1) {
-                        a.front[cur ^ 1][atomicAdd(&cnt[cur ^ 1], 1)] = nb;
+                        (cur ? a.front[0] : a.front[1])[atomicAdd(next, 1)] = nb;
                     }
                 }
             }
-            __syncwarp(gmask);
-        }
-        __syncthreads();  // the round's gradients and the next round are complete
-        if (tid == 0) cnt[cur] = 0;
-        __syncthreads();
+        if (tid == 0) cnt[(r + 2) % 3] = 0;  // last read a barrier ago, next written a barrier on
+        __syncthreads();                     // the round's gradients and the next round are complete
     }
     if (capped) atomicOr(a.flags, (unsigned)kFlagLimiterCapped);
 }
@@ -583,14 +536,24 @@ constexpr int kMaxRounds = 24;  // rounds as launches of their own at most
 
 // the limiter over every flagged cell; `corners`: how many corners are flagged
 void launch_limiter(const LimiterArgs &a, long corners, cudaStream_t s) {
-    const int cx = a.nx - 1, cy = a.ny - 1, cz = a.nz - 1;
+    const int cx = a.nx - 1, cy = a.ny - 1, cz = a.nz == 1 ? 1 : a.nz - 1;
     const long cells = (long)cx * cy * cz;
     if (cells <= kSmallCells) {
         const int cap = most_apart(cx, cy, cz);
-        const size_t smem = (size_t)(cells + 3) / 4 * 8 + (size_t)cap * 4;
-        BINDER_CUDA(cudaFuncSetAttribute(limiter_tail_kernel<true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        count_launch(), limiter_tail_kernel<true><<<1, kTailThreads, smem, s>>>(a, 0, cap);
+        const size_t tables = (size_t)(cells + 3) / 4 * 8 + (size_t)cap * 4;
+        auto launch = [&](auto dim) {
+            constexpr int DIM = decltype(dim)::value;
+            const size_t per = CellGrid<DIM>::kStride * sizeof(double), room = 226 * 1024 - tables;
+            const int groups = room / per < kTailThreads / 4 ? (int)(room / per) : kTailThreads / 4;
+            const size_t smem = groups * per + tables;
+            BINDER_CUDA(cudaFuncSetAttribute(limiter_tail_kernel<DIM, true>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem));
+            count_launch(), limiter_tail_kernel<DIM, true><<<1, kTailThreads, smem, s>>>(a, 0, cap,
+                                                                                        groups);
+        };
+        if (a.nz == 1) launch(std::integral_constant<int, 2>());
+        else launch(std::integral_constant<int, 3>());
         BINDER_CUDA(cudaGetLastError());
         return;
     }
@@ -601,11 +564,16 @@ void launch_limiter(const LimiterArgs &a, long corners, cudaStream_t s) {
     long b = (cells + 255) / 256;
     const int grid = (int)(b < 148L * 16 ? b : 148L * 16);
     count_launch(), limiter_start_kernel<<<grid, 256, 0, s>>>(a);
-    b = (corners + 15) / 16;
+    b = (corners + 63) / 64;
     const int rgrid = (int)(b < 148L * 8 ? b : 148L * 8);
     for (int r = 0; r < rounds; ++r)
-        count_launch(), limiter_round_kernel<<<rgrid, 256, 0, s>>>(a, r);
-    count_launch(), limiter_tail_kernel<false><<<1, kTailThreads, 0, s>>>(a, rounds, 0);
+        count_launch(), limiter_round_kernel<<<rgrid, kRoundThreads, 0, s>>>(a, r);
+    constexpr int kGroups = kTailThreads / 4;
+    const size_t smem = (size_t)kGroups * CellGrid<3>::kStride * sizeof(double);
+    BINDER_CUDA(cudaFuncSetAttribute(limiter_tail_kernel<3, false>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    count_launch(), limiter_tail_kernel<3, false><<<1, kTailThreads, smem, s>>>(a, rounds, 0,
+                                                                               kGroups);
     BINDER_CUDA(cudaGetLastError());
 }
 
@@ -630,11 +598,11 @@ __global__ void divergence_kernel(const double *g, int nx, int ny, int nz, doubl
 }
 
 // topology_correction_2D.cpp:165-207: the 4 corner Jacobians of every cell in the vertex order
-// 00, 10, 01, 11 (the reference's Jff, Jbf, Jfb, Jbb).  Corner (vx, vy) pairs the x edge at
-// y + vy with the y edge at x + vx (hi - lo each).  `below` / `above` count cells with a corner
-// out of range, as the reference's counters do.  Positions are SoA [2][V].
+// 00, 10, 01, 11 (the reference's Jff, Jbf, Jfb, Jbb), as a mask of those out of range.  Corner
+// (vx, vy) pairs the x edge at y + vy with the y edge at x + vx (hi - lo each).  `below` / `above`
+// count cells with a corner out of range, as the reference's counters do.  Positions are SoA [2][V].
 __global__ void corner2d_kernel(const double *pos, int nx, int ny, double vol, double e1,
-                                double e2, double *Jc, Red *red) {
+                                double e2, uint8_t *mask, Red *red) {
     const long V = (long)nx * ny;
     const long cy = ny - 1;
     const long cells = (long)(nx - 1) * cy;
@@ -647,6 +615,7 @@ __global__ void corner2d_kernel(const double *pos, int nx, int ny, double vol, d
         const double Y00 = pos[V + p00], Y01 = pos[V + p00 + 1], Y10 = pos[V + p10],
                      Y11 = pos[V + p10 + 1];
         bool lo = false, hi = false;
+        unsigned bits = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int vx = c & 1, vy = c >> 1;
@@ -654,10 +623,11 @@ __global__ void corner2d_kernel(const double *pos, int nx, int ny, double vol, d
             const double ex0 = vy ? X11 - X01 : X10 - X00, ex1 = vy ? Y11 - Y01 : Y10 - Y00;
             const double ey0 = vx ? X11 - X10 : X01 - X00, ey1 = vx ? Y11 - Y10 : Y01 - Y00;
             const double j = (ex0 * ey1 - ey0 * ex1) * vol;
-            Jc[cell * 4 + c] = j;
             lo |= j < e1;
             hi |= j > e2;
+            bits |= (j < e1 || j > e2) ? 1u << c : 0u;
         }
+        mask[cell] = (uint8_t)bits;
         lb += lo;
         la += hi;
     }
@@ -687,233 +657,6 @@ __global__ void gradient2d_kernel(const double *pos, int nx, int ny, double v0, 
         g[2 * V + p] = (pos[V + px] - c1) / v1;
         g[3 * V + p] = (pos[V + py] - c1) / v1;
     }
-}
-
-__global__ void flag_cells2d_kernel(const double *Jc, int nx, int ny, double e1, double e2,
-                                    int *list, Red *red) {
-    const long cells = (long)(nx - 1) * (ny - 1);
-    for (long cell = (long)blockIdx.x * blockDim.x + threadIdx.x; cell < cells;
-         cell += (long)gridDim.x * blockDim.x) {
-        bool any = false;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const double j = Jc[cell * 4 + c];
-            any |= (j < e1 || j > e2);
-        }
-        if (any) list[atomicAdd(&red->count, 1)] = (int)cell;
-    }
-}
-
-// topology_correction_2D.cpp:248-313.  Cells are visited in lexicographic order and a cell's 4
-// corners in order; a cell touches gradients only at its own 2x2 nodes, so two cells interact
-// only if they differ by at most 1 along both axes.  Level 2x + y orders every such pair as the
-// lexicographic walk does and never puts two of them on one level, so levels in increasing order
-// (cells of one level in parallel) reproduce the sequential result exactly.  Column n2 of a
-// corner's matrix is read at the corner's vertex with its n2 bit cleared, so a corner reads
-// nodes (0, vy) and (vx, 0) of its cell and node (1, 1) is never read.
-//
-// The walk is a chain of some 3 max(nx, ny) short levels, so its time is the chain's length times
-// the latency of one level.  One warp walks (a warp barrier per level), on shared-memory copies:
-// the block first gives every node a flagged corner reads a slot (a V-sized map, -1 between
-// calls), gathers those nodes' gradients and the cells' flagged-corner masks, and afterwards
-// scatters the gradients back.  More than kStageCells cells or kStageNodes nodes: the warp walks
-// global memory.  Either way the arithmetic and its order are those of the sequential walk.
-constexpr int kLimiterThreads = 1024;
-constexpr int kStageCells = 4096;
-constexpr int kStageNodes = 6016;
-// shared bytes of the staged walk: per node 4 gradients, per cell 3 slots and the corner mask
-// (16 bits each)
-constexpr size_t kStageBytes =
-    kStageNodes * 4 * sizeof(double) + kStageCells * 4 * sizeof(unsigned short);
-constexpr unsigned short kNoSlot = 0xffff;
-static_assert(kStageNodes < kNoSlot, "slots are 16-bit");
-
-__global__ void __launch_bounds__(kLimiterThreads) limiter2d_kernel(const int *list, int *sorted,
-                                                                    const double *Jc, double *g,
-                                                                    int nx, int ny, double e1,
-                                                                    double e2, int nlev, Red *red,
-                                                                    unsigned *flags, int *slot) {
-    extern __shared__ __align__(16) unsigned char lsm[];
-    int *off = reinterpret_cast<int *>(lsm);  // nlev + 1
-    int *cur = off + nlev + 1;                // nlev
-    const size_t o = ((size_t)(2 * nlev + 1) * sizeof(int) + 15) & ~(size_t)15;
-    double *gs = reinterpret_cast<double *>(lsm + o);  // [kStageNodes][4]
-    // [kStageCells][4]: slots of nodes (0, 0), (1, 0), (0, 1), then the flagged-corner mask
-    unsigned short *cs = reinterpret_cast<unsigned short *>(gs + (size_t)kStageNodes * 4);
-    __shared__ int nslot;
-    const long V = (long)nx * ny;
-    const long cy = ny - 1;
-    const int n = red->count;
-    const int tid = threadIdx.x, lane = tid & 31;
-    for (int l = tid; l < nlev + 1; l += blockDim.x) off[l] = 0;
-    if (tid == 0) nslot = 0;
-    __syncthreads();
-    for (int q = tid; q < n; q += blockDim.x) {
-        const long cell = list[q];
-        atomicAdd(&off[2 * (int)(cell / cy) + (int)(cell % cy) + 1], 1);
-    }
-    __syncthreads();
-    if (tid == 0)
-        for (int l = 0; l < nlev; ++l) off[l + 1] += off[l];
-    __syncthreads();
-    for (int l = tid; l < nlev; l += blockDim.x) cur[l] = off[l];
-    __syncthreads();
-    for (int q = tid; q < n; q += blockDim.x) {
-        const long cell = list[q];
-        sorted[atomicAdd(&cur[2 * (int)(cell / cy) + (int)(cell % cy)], 1)] = (int)cell;
-    }
-    __syncthreads();
-    bool staged = false;
-    if (n <= kStageCells) {
-        // claim a slot for every node (0, 0), (1, 0), (0, 1) a flagged corner reads
-        for (int q = tid; q < n; q += blockDim.x) {
-            const long cell = sorted[q];
-            const int x = (int)(cell / cy), y = (int)(cell % cy);
-            unsigned m = 0;
-            for (int c = 0; c < 4; ++c) {
-                const double jv = Jc[cell * 4 + c];
-                m |= (jv < e1 || jv > e2) ? 1u << c : 0u;
-            }
-            cs[q * 4 + 3] = (unsigned short)m;
-            const unsigned need = ((m & 1u) ? 1u : 0u) | ((m & 2u) ? 3u : 0u) |
-                                  ((m & 4u) ? 5u : 0u) | ((m & 8u) ? 6u : 0u);  // bit d: node d
-            int old[3];
-            long p[3];
-            for (int d = 0; d < 3; ++d) {
-                p[d] = (long)(x + (d & 1)) * ny + (y + (d >> 1));
-                old[d] = (need >> d & 1u) ? atomicCAS(&slot[p[d]], -1, -2) : 0;
-            }
-            for (int d = 0; d < 3; ++d)
-                if ((need >> d & 1u) && old[d] == -1) {
-                    slot[p[d]] = atomicAdd(&nslot, 1);
-                }
-        }
-        __syncthreads();  // every claimed node holds its slot number
-        const int ns = nslot;
-        if (ns <= kStageNodes) {
-            staged = true;
-            // slots of the cells and the nodes' gradients (a node shared by cells is gathered
-            // once per cell, the same values into the same slot)
-            for (int q = tid; q < n; q += blockDim.x) {
-                const long cell = sorted[q];
-                const int x = (int)(cell / cy), y = (int)(cell % cy);
-                const unsigned m = cs[q * 4 + 3];
-                const unsigned need = ((m & 1u) ? 1u : 0u) | ((m & 2u) ? 3u : 0u) |
-                                      ((m & 4u) ? 5u : 0u) | ((m & 8u) ? 6u : 0u);
-                for (int d = 0; d < 3; ++d) {
-                    unsigned short sl = kNoSlot;
-                    if (need >> d & 1u) {
-                        const long p = (long)(x + (d & 1)) * ny + (y + (d >> 1));
-                        sl = (unsigned short)slot[p];
-                        for (int k = 0; k < 4; ++k) gs[sl * 4 + k] = g[k * V + p];
-                    }
-                    cs[q * 4 + d] = sl;
-                }
-            }
-        } else {
-            // too many nodes: release the map and walk global memory
-            for (int q = tid; q < n; q += blockDim.x) {
-                const long cell = sorted[q];
-                const int x = (int)(cell / cy), y = (int)(cell % cy);
-                for (int d = 0; d < 3; ++d) slot[(long)(x + (d & 1)) * ny + (y + (d >> 1))] = -1;
-            }
-        }
-        __syncthreads();
-    }
-    bool capped = false;
-    if (tid < 32) {
-        // lane gl of a 16-lane group: alpha of trial gl and of the step after it
-        const int grp = lane >> 4, gl = lane & 15;
-        const unsigned gmask = grp ? 0xffff0000u : 0x0000ffffu;
-        double at = 0.0, an = 0.0, a = 0.0;
-        for (int t = 0; t <= 11; ++t) {
-            const double a1 = fmin(a + 0.1, 1.0);  // alpha += 0.1, capped at 1
-            if (t == gl) {
-                at = a;
-                an = a1;
-            }
-            a = a1;
-        }
-        for (int l = 0; l < nlev; ++l) {
-            const int beg = off[l], end = off[l + 1];
-            if (beg == end) continue;  // uniform: every lane reads the same shared value
-            if (staged && end - beg <= 2) {
-                // one or two cells: a group of 16 lanes per cell, the trials across the lanes
-                const int q = beg + grp;
-                if (q < end) {  // uniform across the group
-                    const unsigned m = cs[q * 4 + 3];
-                    for (int c = 0; c < 4; ++c) {
-                        if (!(m >> c & 1u)) continue;
-                        const int vx = c & 1, vy = c >> 1;
-                        const int sv[2] = {cs[q * 4 + 2 * vy], cs[q * 4 + vx]};
-                        double J[2][2];
-                        for (int n1 = 0; n1 < 2; ++n1)
-                            for (int n2 = 0; n2 < 2; ++n2)
-                                J[n1][n2] = gs[sv[n2] * 4 + n1 * 2 + n2];
-                        limit_corner_lanes(J, e1, e2, capped, gl, gmask, at, an);
-                        // every lane stores the same values; each reads its own store back
-                        for (int n1 = 0; n1 < 2; ++n1)
-                            for (int n2 = 0; n2 < 2; ++n2)
-                                gs[sv[n2] * 4 + n1 * 2 + n2] = J[n1][n2];
-                    }
-                }
-                __syncwarp();
-                continue;
-            }
-            for (int q = beg + lane; q < end; q += 32) {
-                if (staged) {
-                    const unsigned m = cs[q * 4 + 3];
-                    for (int c = 0; c < 4; ++c) {
-                        if (!(m >> c & 1u)) continue;
-                        const int vx = c & 1, vy = c >> 1;
-                        const int sv[2] = {cs[q * 4 + 2 * vy], cs[q * 4 + vx]};
-                        double J[2][2];
-                        for (int n1 = 0; n1 < 2; ++n1)
-                            for (int n2 = 0; n2 < 2; ++n2)
-                                J[n1][n2] = gs[sv[n2] * 4 + n1 * 2 + n2];
-                        limit_corner<2>(J, e1, e2, capped);
-                        for (int n1 = 0; n1 < 2; ++n1)
-                            for (int n2 = 0; n2 < 2; ++n2)
-                                gs[sv[n2] * 4 + n1 * 2 + n2] = J[n1][n2];
-                    }
-                } else {
-                    const long cell = sorted[q];
-                    const int x = (int)(cell / cy), y = (int)(cell % cy);
-                    for (int c = 0; c < 4; ++c) {
-                        const double jv = Jc[cell * 4 + c];
-                        if (!(jv < e1 || jv > e2)) continue;
-                        const int vx = c & 1, vy = c >> 1;
-                        const long gp[2] = {(long)x * ny + (y + vy), (long)(x + vx) * ny + y};
-                        double J[2][2];
-                        for (int n1 = 0; n1 < 2; ++n1)
-                            for (int n2 = 0; n2 < 2; ++n2)
-                                J[n1][n2] = g[(n1 * 2 + n2) * V + gp[n2]];
-                        limit_corner<2>(J, e1, e2, capped);
-                        for (int n1 = 0; n1 < 2; ++n1)
-                            for (int n2 = 0; n2 < 2; ++n2)
-                                g[(n1 * 2 + n2) * V + gp[n2]] = J[n1][n2];
-                    }
-                }
-            }
-            __syncwarp();
-        }
-    }
-    if (staged) {
-        __syncthreads();
-        // scatter back (a shared node once per cell, the same values) and release the map
-        for (int q = tid; q < n; q += blockDim.x) {
-            const long cell = sorted[q];
-            const int x = (int)(cell / cy), y = (int)(cell % cy);
-            for (int d = 0; d < 3; ++d) {
-                const unsigned short sl = cs[q * 4 + d];
-                if (sl == kNoSlot) continue;
-                const long p = (long)(x + (d & 1)) * ny + (y + (d >> 1));
-                for (int k = 0; k < 4; ++k) g[k * V + p] = gs[sl * 4 + k];
-                slot[p] = -1;
-            }
-        }
-    }
-    if (capped) atomicOr(flags, (unsigned)kFlagLimiterCapped);
 }
 
 // backward-difference divergence (periodic) of each component's 2D gradient row
@@ -1076,7 +819,6 @@ __global__ void clear_red_kernel(Red *r) {
     r->mx = 0ull;
     r->below = r->above = r->negative = 0ull;
     r->sum[0] = r->sum[1] = r->sum[2] = 0.0;
-    r->count = 0;
     r->pad = 0;
 }
 }  // namespace
@@ -1140,11 +882,10 @@ struct TopologyWorkspace::Impl {
     DBuf<unsigned> flags;
     // allocated when a correction first iterates (most calls find every Jacobian in range)
     bool ready = false;
-    DBuf<double> grad, jc, div, t1, t2;
+    DBuf<double> grad, div, t1, t2;
     DBuf<int> list, sorted;
-    DBuf<uint8_t> mask;  // 3D: flagged corners per cell
+    DBuf<uint8_t> mask;  // flagged corners per cell
     DBuf<int> deg, counts;
-    DBuf<int> slot;  // image node -> shared-memory slot of the 2D limiter, -1 between calls
     HartleyMatrix H[3];
     DBuf<double> cs[3];
     Impl(int x, int y, int z, cudaStream_t s)
@@ -1157,22 +898,16 @@ struct TopologyWorkspace::Impl {
     void ensure() {
         if (ready) return;
         grad.alloc(V * N * N, st);
-        if (nz == 1) {
-            jc.alloc(cells * 4, st);
-        } else {
-            mask.alloc(cells, st);
+        mask.alloc(cells, st);
+        if (cells > kSmallCells) {  // the limiter's rounds in global memory
             deg.alloc(cells, st);
             counts.alloc(kMaxRounds + 1, st);
+            list.alloc(cells, st);
+            sorted.alloc(cells, st);
         }
         div.alloc(V * N, st);
         t1.alloc(V * N, st);
         t2.alloc(V * N, st);
-        list.alloc(cells, st);
-        sorted.alloc(cells, st);
-        if (nz == 1) {
-            slot.alloc(V, st);
-            BINDER_CUDA(cudaMemsetAsync(slot.p, 0xff, sizeof(int) * V, st));
-        }
         const int dims[3] = {nx, ny, nz};
         const double pi = 3.14159265358979323846;
         for (int a = 0; a < 3; ++a) {
@@ -1319,7 +1054,7 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
     auto corners = [&]() {
         reset_red(w.red.p, s);
         count_launch(), corner2d_kernel<<<grid_for(cells), 256, 0, s>>>(w.pos.p, nx, ny, vol, e1,
-                                                                        e2, w.jc.p, w.red.p);
+                                                                        e2, w.mask.p, w.red.p);
         BINDER_CUDA(cudaGetLastError());
         return read_red(w.red.p, s);
     };
@@ -1328,11 +1063,6 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
     double jmin = unordered(r.mn), jmax = unordered(r.mx);
     res.below_before = (long long)r.below;
     res.above_before = (long long)r.above;
-    const int nlev = 2 * (nx - 2) + (ny - 2) + 1;
-    const size_t lim_smem =
-        ((sizeof(int) * (2 * (size_t)nlev + 1) + 15) & ~(size_t)15) + kStageBytes;
-    BINDER_CUDA(cudaFuncSetAttribute(limiter2d_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim_smem));
     int outer = 0;
     while ((jmin < e1 || jmax > e2) && outer < max_outer) {
         w.ensure();
@@ -1342,11 +1072,13 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
             count_launch(), gradient2d_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, nx, ny, vs[0],
                                                                           vs[1], w.grad.p);
             reset_red(w.red.p, s);
-            count_launch(), flag_cells2d_kernel<<<grid_for(cells), 256, 0, s>>>(
-                                w.jc.p, nx, ny, e1, e2, w.list.p, w.red.p);
-            count_launch(), limiter2d_kernel<<<1, kLimiterThreads, lim_smem, s>>>(
-                                w.list.p, w.sorted.p, w.jc.p, w.grad.p, nx, ny, e1, e2, nlev,
-                                w.red.p, w.flags.p, w.slot.p);
+            LimiterArgs la{};
+            la.mask = w.mask.p;
+            la.g = w.grad.p;
+            la.nx = nx; la.ny = ny; la.nz = 1;
+            la.e1 = e1; la.e2 = e2;
+            la.flags = w.flags.p;
+            launch_limiter(la, (long)(c.below + c.above), s);
             BINDER_CUDA(cudaGetLastError());
             count_launch(), sum_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, V, 2, w.red.p);
             count_launch(), divergence2d_kernel<<<grid_for(V), 256, 0, s>>>(w.grad.p, nx, ny,
