@@ -6,9 +6,9 @@
 // k = 0 .. n/2 give H[k] = C_k + S_k and H[n-k] = C_k - S_k: two products of (n/2)^2 instead of one
 // of n^2, half the operations.
 //
-// A CTA of four warps owns 32 lines.  It folds them into shared memory (e and o, [j][32] with a
-// pitch of 36 doubles: the four rows of a fragment are 8 banks apart), and warp w computes the
-// 8-row tiles w, w + 4, ... of both products for all 32 lines with mma.m8n8k4 (FP64 in, FP64 FMA
+// A CTA of four warps owns 32 (or 8) lines.  It folds them into shared memory (e and o, [j][32] with
+// a pitch of 36 doubles, or [j][8] with 12: the four rows of a fragment are 8 banks apart), and warp
+// w computes the 8-row tiles w, w + 4, ... of both products for all its lines with mma.m8n8k4 (FP64 in, FP64 FMA
 // accumulation), the matrices coming from global memory through L1.  kHartleyPoisson folds the
 // scaled coefficients straight from the accumulators -- a thread holds k and n - k of its lines --
 // and transforms again, so the spectrum is never stored.
@@ -18,7 +18,8 @@
 // 0.34 ms, where a 64-line register-blocked FMA kernel of the unfolded matrix took 0.6 / 0.95 / 0.95
 // (one CTA of eight warps per SM, its staging not overlapped, a division per staged element).
 // 32 lines and four warps per CTA, so that two or three CTAs share an SM and one's folding overlaps
-// another's products.
+// another's products; 8 lines where 32 would leave SMs without a CTA (two components at
+// 128x128, y / x with the Poisson scaling / y: 14.6 / 29.0 / 14.8 us with 32 lines, 6.4 / 11.1 / 6.6 with 8).
 #include <cmath>
 #include <vector>
 
@@ -28,9 +29,12 @@
 namespace binder {
 namespace {
 
-constexpr int kLinesH = 32;  // lines per CTA
-constexpr int kPitchH = 36;  // doubles per row of e / o
 constexpr int kThreadsH = 128;
+// LT: 8-line tiles of a CTA (4 or 1)
+template <int LT>
+constexpr int kLinesH = 8 * LT;
+template <int LT>
+constexpr int kPitchH = 8 * LT + 4;  // doubles per row of e / o
 
 struct HArgs {
     HartleyArgs a;
@@ -46,14 +50,14 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 }
 
 // both products of this warp's tiles: cC = cos e, cS = sin o
-template <int U>
+template <int U, int LT>
 __device__ __forceinline__ void products(const HArgs &h, const double *E, const double *O,
-                                         double (&cC)[U][4][2], double (&cS)[U][4][2], int warp,
+                                         double (&cC)[U][LT][2], double (&cS)[U][LT][2], int warp,
                                          int lane) {
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int t = 0; t < 4; ++t) cC[u][t][0] = cC[u][t][1] = cS[u][t][0] = cS[u][t][1] = 0.0;
+        for (int t = 0; t < LT; ++t) cC[u][t][0] = cC[u][t][1] = cS[u][t][0] = cS[u][t][1] = 0.0;
     const int ar = lane >> 2, ak = lane & 3;
     const double *pc[U], *ps[U];
 #pragma unroll
@@ -71,9 +75,9 @@ __device__ __forceinline__ void products(const HArgs &h, const double *E, const 
         const int jn = j + 4 < h.cols ? j + 4 : j;
 #pragma unroll
         for (int u = 0; u < U; ++u) n0[u] = __ldg(pc[u] + jn), n1[u] = __ldg(ps[u] + jn);
-        const double *e = E + (j + ak) * kPitchH + ar, *o = O + (j + ak) * kPitchH + ar;
+        const double *e = E + (j + ak) * kPitchH<LT> + ar, *o = O + (j + ak) * kPitchH<LT> + ar;
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
+        for (int t = 0; t < LT; ++t) {
             const double be = e[t * 8], bo = o[t * 8];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -86,10 +90,11 @@ __device__ __forceinline__ void products(const HArgs &h, const double *E, const 
     }
 }
 
-template <int U, int MODE>
+template <int U, int MODE, int LT>
 __global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(const HArgs h) {
+    constexpr int kLines = kLinesH<LT>, kPitch = kPitchH<LT>;
     extern __shared__ __align__(16) double sm[];
-    double *E = sm, *O = sm + (long)h.cols * kPitchH;
+    double *E = sm, *O = sm + (long)h.cols * kPitch;
     const HartleyArgs &a = h.a;
     const int n = h.n, half = n >> 1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int comp = blockIdx.y;
@@ -100,22 +105,23 @@ __global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(cons
     int nl;     // lines of the tile
     long t0 = 0;
     if (contig) {
-        const long l0 = (long)blockIdx.x * kLinesH;
-        nl = (int)min((long)kLinesH, a.outer - l0);
+        const long l0 = (long)blockIdx.x * kLines;
+        nl = (int)min((long)kLines, a.outer - l0);
         base = l0 * n;
     } else {
-        const long tiles = (a.s + kLinesH - 1) / kLinesH;
+        const long tiles = (a.s + kLines - 1) / kLines;
         const long o = blockIdx.x / tiles;
-        t0 = (blockIdx.x - o * tiles) * kLinesH;
-        nl = (int)min((long)kLinesH, a.s - t0);
+        t0 = (blockIdx.x - o * tiles) * kLines;
+        nl = (int)min((long)kLines, a.s - t0);
         base = o * n * a.s + t0;
     }
     const long js = contig ? 1 : a.s, ls = contig ? n : 1;  // strides of j and of the lines
     // ---- fold: contiguous lines 8 j x 4 lines per warp instruction (64-byte segments), strided
-    // ones 32 neighbouring lines
-    const int lj = contig ? lane & 7 : 0, ll = contig ? lane >> 3 : lane;
-    for (int c0 = 0; c0 < kLinesH; c0 += contig ? 4 : kLinesH)
-        for (int j = (contig ? warp * 8 : warp) + lj; j < h.cols; j += contig ? 32 : 4) {
+    // ones all the neighbouring lines (x 4 j for 8 lines)
+    const int wj = contig ? 8 : 32 / kLines;  // j per warp instruction
+    const int lj = contig ? lane & 7 : lane / kLines, ll = contig ? lane >> 3 : lane % kLines;
+    for (int c0 = 0; c0 < kLines; c0 += contig ? 4 : kLines)
+        for (int j = warp * wj + lj; j < h.cols; j += 4 * wj) {
             const int c = c0 + ll;
             double e = 0.0, o = 0.0;
             if (c < nl && j <= half) {
@@ -129,19 +135,19 @@ __global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(cons
                     o = x - y;
                 }
             }
-            E[j * kPitchH + c] = e;
-            O[j * kPitchH + c] = o;
+            E[j * kPitch + c] = e;
+            O[j * kPitch + c] = o;
         }
     __syncthreads();
-    double cC[U][4][2], cS[U][4][2];
-    products<U>(h, E, O, cC, cS, warp, lane);
+    double cC[U][LT][2], cS[U][LT][2];
+    products<U, LT>(h, E, O, cC, cS, warp, lane);
     // this thread's rows k = 8 m + lane / 4 and lines t * 8 + 2 (lane % 4) + {0, 1}
     const int kr = lane >> 2, lc = (lane & 3) * 2;
     if (MODE == kHartleyPoisson) {
         __syncthreads();  // every warp has read e and o
         const double inv_total = 1.0 / ((double)n * (double)a.s);
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
+        for (int t = 0; t < LT; ++t)
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int c = t * 8 + lc + q;
@@ -163,22 +169,22 @@ __global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(cons
                         o = e - y;
                         e = e + y;
                     }
-                    E[k * kPitchH + c] = e;
-                    O[k * kPitchH + c] = o;
+                    E[k * kPitch + c] = e;
+                    O[k * kPitch + c] = o;
                 }
             }
         __syncthreads();
-        products<U>(h, E, O, cC, cS, warp, lane);
+        products<U, LT>(h, E, O, cC, cS, warp, lane);
     }
     const double sc = MODE == kHartleyScaled ? a.out_scale[comp] : 1.0;
-    const double of = MODE == kHartleyScaled ? a.out_offset[comp] : 0.0;
+    const double of = MODE == kHartleyScaled ? a.sums[comp] / a.count : 0.0;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const int k = (warp + 4 * u) * 8 + kr;
         if (warp + 4 * u >= h.tiles || k > half) continue;
         const bool pair = k != 0 && 2 * k != n;
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
+        for (int t = 0; t < LT; ++t)
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int c = t * 8 + lc + q;
@@ -192,17 +198,30 @@ __global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(cons
     }
 }
 
+long line_tiles(const HartleyArgs &a, int lines) {
+    return a.s == 1 ? (a.outer + lines - 1) / lines : a.outer * ((a.s + lines - 1) / lines);
+}
+
+template <int U, int MODE, int LT>
+void launch_l(const HArgs &h, int ncomp, cudaStream_t s) {
+    const size_t smem = (size_t)2 * h.cols * kPitchH<LT> * sizeof(double);
+    BINDER_CUDA(cudaFuncSetAttribute(hartley_kernel<U, MODE, LT>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const long gx = line_tiles(h.a, kLinesH<LT>);
+    BINDER_CHECK(gx < (1L << 31), "transform grid too large");
+    count_launch(), hartley_kernel<U, MODE, LT>
+        <<<dim3((unsigned)gx, (unsigned)ncomp), kThreadsH, smem, s>>>(h);
+    BINDER_CUDA(cudaGetLastError());
+}
+
+// 8 lines per CTA where 32 make fewer CTAs than SMs
 template <int U, int MODE>
 void launch_u(const HArgs &h, int ncomp, cudaStream_t s) {
-    const size_t smem = (size_t)2 * h.cols * kPitchH * sizeof(double);
-    BINDER_CUDA(cudaFuncSetAttribute(hartley_kernel<U, MODE>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const long gx = h.a.s == 1 ? (h.a.outer + kLinesH - 1) / kLinesH
-                               : h.a.outer * ((h.a.s + kLinesH - 1) / kLinesH);
-    BINDER_CHECK(gx < (1L << 31), "transform grid too large");
-    count_launch(), hartley_kernel<U, MODE><<<dim3((unsigned)gx, (unsigned)ncomp), kThreadsH, smem,
-                                             s>>>(h);
-    BINDER_CUDA(cudaGetLastError());
+    int dev = 0, sms = 148;
+    BINDER_CUDA(cudaGetDevice(&dev));
+    BINDER_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (line_tiles(h.a, kLinesH<4>) * ncomp < sms) launch_l<U, MODE, 1>(h, ncomp, s);
+    else launch_l<U, MODE, 4>(h, ncomp, s);
 }
 
 template <int MODE>

@@ -16,7 +16,7 @@ struct HartleyMatrix {
 
 enum HartleyMode : int {
     kHartleyPlain = 0,    // y = H x
-    kHartleyScaled = 1,   // y = (H x) * out_scale + out_offset, per component
+    kHartleyScaled = 1,   // y = (H x) * out_scale + sums / count, per component
     kHartleyPoisson = 2,  // y = H (-(H x) / (lambda V)) along the outermost axis (outer == 1)
 };
 
@@ -27,7 +27,9 @@ struct HartleyArgs {
     long outer, s;     // element (o, j, t) of the axis at o * n * s + j * s + t
     int nz;            // kHartleyPoisson: t = ky * nz + kz
     const double *cos_x, *cos_y, *cos_z;  // cos(2 pi k / n) per axis
-    double out_scale[3], out_offset[3];
+    double out_scale[3];
+    const double *sums;  // on the device: the offset is a mean that no host needs to know
+    double count;
 };
 
 // One pass over `ncomp` components along the axis of H (at most 256 long).

@@ -972,7 +972,6 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
         while ((c.below > 0 || c.above > 0) && inner < max_inner) {
             count_launch(), gradient_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, nx, ny, nz, vs[0], vs[1], vs[2],
                                                         w.grad.p);
-            reset_red(w.red.p, s);
             LimiterArgs la{};
             la.mask = w.mask.p;
             la.g = w.grad.p;
@@ -985,12 +984,10 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
             la.flags = w.flags.p;
             launch_limiter(la, (long)(c.below + c.above), s);
             BINDER_CUDA(cudaGetLastError());
+            // the mean position, from the zeros that corners() left
             count_launch(), sum_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, V, 3, w.red.p);
             count_launch(), divergence_kernel<<<grid_for(V), 256, 0, s>>>(w.grad.p, nx, ny, nz, w.div.p);
             BINDER_CUDA(cudaGetLastError());
-            Red sr = read_red(w.red.p, s);
-            double mean[3];
-            for (int n = 0; n < 3; ++n) mean[n] = sr.sum[n] / (nx * ny * nz);
 
             // u = -(1/V) H (H div / lambda): separable Hartley passes z, y, [x fused], y, z
             HartleyArgs a{};
@@ -1009,10 +1006,9 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
             launch_hartley(a, w.H[1], kHartleyPlain, 3, s);
             // last pass: physical positions u * vs + mean
             a.in = w.t2.p; a.out = w.pos.p; a.outer = (long)nx * ny; a.s = 1;
-            for (int n = 0; n < 3; ++n) {
-                a.out_scale[n] = vs[n];
-                a.out_offset[n] = mean[n];
-            }
+            for (int n = 0; n < 3; ++n) a.out_scale[n] = vs[n];
+            a.sums = w.red.p->sum;
+            a.count = nx * ny * nz;
             launch_hartley(a, w.H[2], kHartleyScaled, 3, s);
             c = corners();
             inner++;
@@ -1024,7 +1020,6 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
         outer++;
     }
     res.outer_iterations = outer;
-    r = jac_stats();
     res.below_after = (long long)r.below;
     res.above_after = (long long)r.above;
     BINDER_CUDA(cudaMemcpyAsync(&res.flags, w.flags.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -1071,7 +1066,6 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
         while ((c.below > 0 || c.above > 0) && inner < max_inner) {
             count_launch(), gradient2d_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, nx, ny, vs[0],
                                                                           vs[1], w.grad.p);
-            reset_red(w.red.p, s);
             LimiterArgs la{};
             la.mask = w.mask.p;
             la.g = w.grad.p;
@@ -1080,13 +1074,11 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
             la.flags = w.flags.p;
             launch_limiter(la, (long)(c.below + c.above), s);
             BINDER_CUDA(cudaGetLastError());
+            // the mean position, from the zeros that corners() left
             count_launch(), sum_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, V, 2, w.red.p);
             count_launch(), divergence2d_kernel<<<grid_for(V), 256, 0, s>>>(w.grad.p, nx, ny,
                                                                             w.div.p);
             BINDER_CUDA(cudaGetLastError());
-            Red sr = read_red(w.red.p, s);
-            double mean[2];
-            for (int n = 0; n < 2; ++n) mean[n] = sr.sum[n] / (nx * ny);
 
             // u = -(1/V) H (H div / lambda) on the nx x ny grid (the volume nx x ny x 1, whose
             // unit z axis contributes cos 0 = 1 to lambda = 6 - 2cos_x - 2cos_y - 2cos_z)
@@ -1102,10 +1094,9 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
             launch_hartley(a, w.H[0], kHartleyPoisson, 2, s);
             // last pass: physical positions u * vs + mean
             a.in = w.t2.p; a.out = w.pos.p; a.outer = nx; a.s = 1;
-            for (int n = 0; n < 2; ++n) {
-                a.out_scale[n] = vs[n];
-                a.out_offset[n] = mean[n];
-            }
+            for (int n = 0; n < 2; ++n) a.out_scale[n] = vs[n];
+            a.sums = w.red.p->sum;
+            a.count = nx * ny;
             launch_hartley(a, w.H[1], kHartleyScaled, 2, s);
             c = corners();
             inner++;
@@ -1117,7 +1108,6 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
         outer++;
     }
     res.outer_iterations = outer;
-    r = jac_stats();
     res.below_after = (long long)r.below;
     res.above_after = (long long)r.above;
     BINDER_CUDA(cudaMemcpyAsync(&res.flags, w.flags.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
