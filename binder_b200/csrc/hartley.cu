@@ -6,20 +6,27 @@
 // k = 0 .. n/2 give H[k] = C_k + S_k and H[n-k] = C_k - S_k: two products of (n/2)^2 instead of one
 // of n^2, half the operations.
 //
-// A CTA of four warps owns 32 (or 8) lines.  It folds them into shared memory (e and o, [j][32] with
-// a pitch of 36 doubles, or [j][8] with 12: the four rows of a fragment are 8 banks apart), and warp
-// w computes the 8-row tiles w, w + 4, ... of both products for all its lines with mma.m8n8k4 (FP64 in, FP64 FMA
+// A CTA owns 32 (or 8) lines.  It folds them into shared memory (e and o, [j][32] with a pitch of 36
+// doubles, or [j][8] with 12: the four rows of a fragment are 8 banks apart), and each warp computes
+// its 8-row tiles of both products for all the lines with mma.m8n8k4 (FP64 in, FP64 FMA
 // accumulation), the matrices coming from global memory through L1.  kHartleyPoisson folds the
 // scaled coefficients straight from the accumulators -- a thread holds k and n - k of its lines --
 // and transforms again, so the spectrum is never stored.
 //
 // Bound: the FP64 pipe (0.5 n FMA per element and pass; 5.1 GFLOP per pass at 160x192x160, 0.14 ms at
-// 36 TFLOP/s).  Three components at 160x192x160, z / y / x with the Poisson scaling: 0.21 / 0.29 /
-// 0.34 ms, where a 64-line register-blocked FMA kernel of the unfolded matrix took 0.6 / 0.95 / 0.95
-// (one CTA of eight warps per SM, its staging not overlapped, a division per staged element).
-// 32 lines and four warps per CTA, so that two or three CTAs share an SM and one's folding overlaps
-// another's products; 8 lines where 32 would leave SMs without a CTA (two components at
-// 128x128, y / x with the Poisson scaling / y: 14.6 / 29.0 / 14.8 us with 32 lines, 6.4 / 11.1 / 6.6 with 8).
+// 36 TFLOP/s).  Three components at 160x192x160, z / y / x with the Poisson scaling / y / z back:
+// 0.18 / 0.21 / 0.34 / 0.21 / 0.19 ms, where a 64-line register-blocked FMA kernel of the unfolded
+// matrix took 0.6 / 0.95 / 0.95 / 0.95 / 0.6 (one CTA of eight warps per SM, its staging not
+// overlapped, a division per staged element).
+//
+// A CTA owns 32 lines and has a warp for every two 8-row tiles of the halves (17 tiles at most, at
+// n = 256), so no warp idles but for an odd last tile, and two or three CTAs share an SM, one's
+// folding overlapping another's products.  Four warps with three or four tiles each took 0.21 / 0.29
+// / 0.34 / 0.29 / 0.21: 13 tiles leave three of 16 slots empty.  96 registers are what keeps three CTAs of
+// six warps (or of seven) on an SM; with 128 the passes are 10 to 15 % slower, with 80 (three CTAs
+// asked for of seven warps) 30 %.  Where 32 lines would leave SMs without a CTA, a CTA owns 8 lines
+// and has a warp per tile (two components at 128x128, y / x with the Poisson scaling / y back: 4.4 /
+// 6.8 / 4.4 us, against 14.6 / 29.0 / 14.8 with 32 lines).
 #include <cmath>
 #include <vector>
 
@@ -29,7 +36,6 @@
 namespace binder {
 namespace {
 
-constexpr int kThreadsH = 128;
 // LT: 8-line tiles of a CTA (4 or 1)
 template <int LT>
 constexpr int kLinesH = 8 * LT;
@@ -53,7 +59,7 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 template <int U, int LT>
 __device__ __forceinline__ void products(const HArgs &h, const double *E, const double *O,
                                          double (&cC)[U][LT][2], double (&cS)[U][LT][2], int warp,
-                                         int lane) {
+                                         int nw, int lane) {
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -63,7 +69,7 @@ __device__ __forceinline__ void products(const HArgs &h, const double *E, const 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         // tiles past the last one repeat it: their results are not stored
-        const int m = min(warp + 4 * u, h.tiles - 1);
+        const int m = min(warp + nw * u, h.tiles - 1);
         pc[u] = h.cs + (long)(m * 8 + ar) * h.cols + ak;
         ps[u] = h.sn + (long)(m * 8 + ar) * h.cols + ak;
     }
@@ -90,13 +96,16 @@ __device__ __forceinline__ void products(const HArgs &h, const double *E, const 
     }
 }
 
-template <int U, int MODE, int LT>
-__global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(const HArgs h) {
+// U: 8-row tiles per warp; W: warps of a CTA at most (a warp for every U tiles); CTAS: to an SM
+template <int U, int MODE, int LT, int W, int CTAS>
+__global__ void __launch_bounds__(32 * W, CTAS)
+    hartley_kernel(const HArgs h) {
     constexpr int kLines = kLinesH<LT>, kPitch = kPitchH<LT>;
     extern __shared__ __align__(16) double sm[];
     double *E = sm, *O = sm + (long)h.cols * kPitch;
     const HartleyArgs &a = h.a;
     const int n = h.n, half = n >> 1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nw = blockDim.x >> 5;
     const int comp = blockIdx.y;
     const double *in = a.in + comp * a.V;
     double *out = a.out + comp * a.V;
@@ -121,7 +130,7 @@ __global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(cons
     const int wj = contig ? 8 : 32 / kLines;  // j per warp instruction
     const int lj = contig ? lane & 7 : lane / kLines, ll = contig ? lane >> 3 : lane % kLines;
     for (int c0 = 0; c0 < kLines; c0 += contig ? 4 : kLines)
-        for (int j = warp * wj + lj; j < h.cols; j += 4 * wj) {
+        for (int j = warp * wj + lj; j < h.cols; j += nw * wj) {
             const int c = c0 + ll;
             double e = 0.0, o = 0.0;
             if (c < nl && j <= half) {
@@ -140,7 +149,7 @@ __global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(cons
         }
     __syncthreads();
     double cC[U][LT][2], cS[U][LT][2];
-    products<U, LT>(h, E, O, cC, cS, warp, lane);
+    products<U, LT>(h, E, O, cC, cS, warp, nw, lane);
     // this thread's rows k = 8 m + lane / 4 and lines t * 8 + 2 (lane % 4) + {0, 1}
     const int kr = lane >> 2, lc = (lane & 3) * 2;
     if (MODE == kHartleyPoisson) {
@@ -160,8 +169,8 @@ __global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(cons
                 };
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int k = (warp + 4 * u) * 8 + kr;
-                    if (warp + 4 * u >= h.tiles || k > half) continue;
+                    const int k = (warp + nw * u) * 8 + kr;
+                    if (warp + nw * u >= h.tiles || k > half) continue;
                     const double C = cC[u][t][q], S = cS[u][t][q];
                     double e = scale(C + S, k), o = 0.0;
                     if (k != 0 && 2 * k != n) {
@@ -174,14 +183,14 @@ __global__ void __launch_bounds__(kThreadsH, U <= 3 ? 3 : 2) hartley_kernel(cons
                 }
             }
         __syncthreads();
-        products<U, LT>(h, E, O, cC, cS, warp, lane);
+        products<U, LT>(h, E, O, cC, cS, warp, nw, lane);
     }
     const double sc = MODE == kHartleyScaled ? a.out_scale[comp] : 1.0;
     const double of = MODE == kHartleyScaled ? a.sums[comp] / a.count : 0.0;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-        const int k = (warp + 4 * u) * 8 + kr;
-        if (warp + 4 * u >= h.tiles || k > half) continue;
+        const int k = (warp + nw * u) * 8 + kr;
+        if (warp + nw * u >= h.tiles || k > half) continue;
         const bool pair = k != 0 && 2 * k != n;
 #pragma unroll
         for (int t = 0; t < LT; ++t)
@@ -202,37 +211,27 @@ long line_tiles(const HartleyArgs &a, int lines) {
     return a.s == 1 ? (a.outer + lines - 1) / lines : a.outer * ((a.s + lines - 1) / lines);
 }
 
-template <int U, int MODE, int LT>
+template <int U, int MODE, int LT, int W, int CTAS>
 void launch_l(const HArgs &h, int ncomp, cudaStream_t s) {
     const size_t smem = (size_t)2 * h.cols * kPitchH<LT> * sizeof(double);
-    BINDER_CUDA(cudaFuncSetAttribute(hartley_kernel<U, MODE, LT>,
+    BINDER_CUDA(cudaFuncSetAttribute(hartley_kernel<U, MODE, LT, W, CTAS>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long gx = line_tiles(h.a, kLinesH<LT>);
     BINDER_CHECK(gx < (1L << 31), "transform grid too large");
-    count_launch(), hartley_kernel<U, MODE, LT>
-        <<<dim3((unsigned)gx, (unsigned)ncomp), kThreadsH, smem, s>>>(h);
+    count_launch(), hartley_kernel<U, MODE, LT, W, CTAS>
+        <<<dim3((unsigned)gx, (unsigned)ncomp), 32 * ((h.tiles + U - 1) / U), smem, s>>>(h);
     BINDER_CUDA(cudaGetLastError());
 }
 
-// 8 lines per CTA where 32 make fewer CTAs than SMs
-template <int U, int MODE>
-void launch_u(const HArgs &h, int ncomp, cudaStream_t s) {
+// 8 lines and a tile per warp where CTAs of 32 lines would be fewer than SMs
+template <int MODE>
+void launch_mode_h(const HArgs &h, int ncomp, cudaStream_t s) {
     int dev = 0, sms = 148;
     BINDER_CUDA(cudaGetDevice(&dev));
     BINDER_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (line_tiles(h.a, kLinesH<4>) * ncomp < sms) launch_l<U, MODE, 1>(h, ncomp, s);
-    else launch_l<U, MODE, 4>(h, ncomp, s);
-}
-
-template <int MODE>
-void launch_mode_h(const HArgs &h, int ncomp, cudaStream_t s) {
-    switch ((h.tiles + 3) / 4) {
-        case 1: launch_u<1, MODE>(h, ncomp, s); break;
-        case 2: launch_u<2, MODE>(h, ncomp, s); break;
-        case 3: launch_u<3, MODE>(h, ncomp, s); break;
-        case 4: launch_u<4, MODE>(h, ncomp, s); break;
-        default: launch_u<5, MODE>(h, ncomp, s); break;
-    }
+    if (line_tiles(h.a, kLinesH<4>) * ncomp < sms) launch_l<1, MODE, 1, 17, 1>(h, ncomp, s);
+    else if (h.tiles <= 12) launch_l<2, MODE, 4, 6, 3>(h, ncomp, s);
+    else launch_l<2, MODE, 4, 9, 2>(h, ncomp, s);
 }
 
 }  // namespace

@@ -35,3 +35,14 @@ def test_volumes(core, oracle, shape, rms, lo, hi):
     want, outer = oracle.topology3d(f, lo, hi, 1, 2, VS, shape)
     assert tc.last_stats["outer_iterations"] == outer
     np.testing.assert_allclose(got.ravel(), want, rtol=0, atol=1e-9)
+
+
+@pytest.mark.parametrize("shape", [(256, 41, 42), (43, 200, 40), (41, 42, 223), (44, 192, 43)])
+def test_hartley_forms(core, oracle, shape):
+    """Axes of 13 to 17 row tiles on grids with a CTA of 32 lines for every SM."""
+    f = field(shape, 0.62, 3.0, sum(shape))
+    tc = core.topology_correction_3D()
+    got = tc.correct_topology(f, 0.05, 20.0, 1, 1, 1, VS, *shape)
+    want, outer = oracle.topology3d(f, 0.05, 20.0, 1, 1, VS, shape)
+    assert tc.last_stats["outer_iterations"] == outer
+    np.testing.assert_allclose(got.ravel(), want, rtol=0, atol=1e-9)
