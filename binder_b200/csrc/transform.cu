@@ -294,28 +294,31 @@ const std::vector<double> &dct2_matrix(int n) {
 }
 
 namespace {
-__global__ void prior_noise_kernel(float *noise, long V, int ncomp, int chain_comps,
+// Bound by issue (two Philox draws of ten rounds, a logarithm and a sine / cosine pair each for
+// three values), so no division per coefficient: a row of CTAs per chain, 32-bit indices (V < 2^31).
+// 32 chains of 96^3, three components: 325 us with a 64-bit division, 263 without (and 286 with
+// 64-bit products in the rounds).
+__global__ void prior_noise_kernel(float *noise, long V, int per, int chains, int multi,
                                    uint64_t seed, uint32_t chain0, const DevState *st,
                                    const int *skip) {
     if (skip && *skip) return;
-    const int per = chain_comps ? chain_comps : ncomp;  // components per chain
-    const int chains = ncomp / per;
-    for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < V * chains;
-         q += (long)gridDim.x * blockDim.x) {
-        const int ch = (int)(q / V);
-        const uint32_t i = (uint32_t)(q - (long)ch * V);
-        const uint32_t sweep = (uint32_t)st[chain_comps ? ch : 0].sweep;
-        const uint32_t chain = chain0 + (uint32_t)(chain_comps ? ch : 0);
-        float *out = noise + (long)ch * per * V + i;
-        // components 0 and 1: the cosine and the sine of one Box-Muller pair (tag 2)
-        const u32x4 r = philox_draw(seed, i, sweep, 2u, chain);
-        const float u1 = u01_f24(r.x), u2 = u01_f24(r.y);
-        const float rad = sqrtf(-2.0f * logf(u1));
-        float sn, cs;
-        sincospif(2.0f * u2, &sn, &cs);
-        out[0] = rad * cs;
-        if (per > 1) out[V] = rad * sn;
-        if (per > 2) out[2 * V] = dct_prior_normal(seed, i, sweep, chain, 2);
+    for (int ch = blockIdx.y; ch < chains; ch += gridDim.y) {
+        const uint32_t sweep = (uint32_t)st[multi ? ch : 0].sweep;
+        const uint32_t chain = chain0 + (uint32_t)ch;
+        float *const row = noise + (long)ch * per * V;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (uint32_t)V;
+             i += gridDim.x * blockDim.x) {
+            float *out = row + i;
+            // components 0 and 1: the cosine and the sine of one Box-Muller pair (tag 2)
+            const u32x4 r = philox_draw(seed, i, sweep, 2u, chain);
+            const float u1 = u01_f24(r.x), u2 = u01_f24(r.y);
+            const float rad = sqrtf(-2.0f * logf(u1));
+            float sn, cs;
+            sincospif(2.0f * u2, &sn, &cs);
+            out[0] = rad * cs;
+            if (per > 1) out[V] = rad * sn;
+            if (per > 2) out[2 * V] = dct_prior_normal(seed, i, sweep, chain, 2);
+        }
     }
 }
 }  // namespace
@@ -324,10 +327,14 @@ void launch_prior_noise(float *noise, long V, int ncomp, int chain_comps, uint64
                         uint32_t chain, const DevState *st, const int *skip, cudaStream_t s) {
     const int per = chain_comps ? chain_comps : ncomp;
     BINDER_CHECK(per >= 1 && per <= 3 && ncomp % per == 0, "noise components");
-    long b = (V * (ncomp / per) + 255) / 256;
-    b = b < 1 ? 1 : (b > 148L * 16 ? 148L * 16 : b);
-    count_launch(), prior_noise_kernel<<<(int)b, 256, 0, s>>>(noise, V, ncomp, chain_comps, seed,
-                                                             chain, st, skip);
+    BINDER_CHECK(V < (1L << 31), "volume too large");
+    const int chains = ncomp / per;
+    // some sixteen CTAs to an SM over all chains
+    const long y = chains < 65535 ? chains : 65535, most = (148L * 16 + y - 1) / y;
+    long x = (V + 255) / 256;
+    x = x < 1 ? 1 : (x > most ? most : x);
+    count_launch(), prior_noise_kernel<<<dim3((unsigned)x, (unsigned)y), 256, 0, s>>>(
+                        noise, V, per, chains, chain_comps ? 1 : 0, seed, chain, st, skip);
     BINDER_CUDA(cudaGetLastError());
 }
 
