@@ -1991,9 +1991,18 @@ void launch_estep(const EStepArgs &args, bool sample, int grid, cudaStream_t s, 
     BINDER_CHECK(chains >= 1 && chains <= 65535 && (chains == 1 || (sample && !a.logt)),
                  "a batch of chains runs the sampling E-step of the MI likelihood only");
     if (chains > 1) {
-        // the single-chain grid (one wave of CTAs) shared out over the chains, rounded down so all
-        // of them are resident at once (every CTA loops over its chain's voxels)
-        const int gx = grid / chains > 0 ? grid / chains : 1;
+        // one to four waves of the single-chain grid (one wave of CTAs) shared out over the chains,
+        // rounded down to the same count for each (every CTA loops over its chain's voxels): the
+        // fewest rounds of voxels to a thread, with two for a CTA's start and merge.  32 chains of
+        // 96^3: 1151 us with one wave (13 CTAs to a chain, 28 of 444 slots idle), 1124 with four (55).
+        int gx = 1;
+        long best = -1;
+        for (int w = 1; w <= 4; ++w) {
+            const long g = (long)w * grid / chains;
+            if (g < 1) continue;
+            const long rounds = w * (ceil_div(a.V, g * kEThreads) + 2L);
+            if (best < 0 || rounds < best) best = rounds, gx = (int)g;
+        }
         const dim3 g2((unsigned)gx, (unsigned)chains, 1);
         if (a.dim == 3)
             count_launch(), estep_kernel<true, 3><<<g2, kEThreads, smem, s>>>(a);
