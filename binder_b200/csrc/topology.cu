@@ -216,28 +216,46 @@ __global__ void corner_kernel(const double *pos, int nx, int ny, int nz, double 
     }
 }
 
+// red->sum[n] += the CTA's s[n]; every thread of the CTA
+template <int N>
+__device__ __forceinline__ void add_sums(double (&s)[N], Red *red) {
+    __shared__ double part[32];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const double v = block_sum(s[n], part);
+        if (threadIdx.x == 0) atomicAdd(&red->sum[n], v);
+    }
+}
+
 // topology_correction_3D.cpp:172-245: periodic forward differences, g[(n1*3+n2)][p] =
-// (pos_n1(p + e_n2) - pos_n1(p)) / vs[n1]
+// (pos_n1(p + e_n2) - pos_n1(p)) / vs[n1], and the sums of the positions into red.  32-bit indices
+// // (V <= 2^24).  EXACT: every vs is a power of two, so the products with the reciprocals (v0 .. v2) are
+// the quotients to the bit.  Bound by DRAM, with the nine FP64 divisions a voxel by those.
+// 160x192x160: 126 us with 64-bit indices, and 71 for the sums in a kernel of their own; now 121
+// together, 85 without the divisions.
+template <bool EXACT>
 __global__ void gradient_kernel(const double *pos, int nx, int ny, int nz, double v0, double v1,
-                                double v2, double *g) {
-    const long V = (long)nx * ny * nz;
+                                double v2, double *g, Red *red) {
+    const unsigned V = (unsigned)nx * ny * nz;
     const double vs[3] = {v0, v1, v2};
-    for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < V;
-         p += (long)gridDim.x * blockDim.x) {
-        const int x = (int)(p / ((long)ny * nz)), y = (int)((p / nz) % ny), z = (int)(p % nz);
-        const int x2 = x + 1 > nx - 1 ? x + 1 - nx : x + 1;
-        const int y2 = y + 1 > ny - 1 ? y + 1 - ny : y + 1;
-        const int z2 = z + 1 > nz - 1 ? z + 1 - nz : z + 1;
-        const long px = ((long)x2 * ny + y) * nz + z, py = ((long)x * ny + y2) * nz + z,
-                   pz = ((long)x * ny + y) * nz + z2;
+    double s[3] = {0.0, 0.0, 0.0};
+    for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < V; p += gridDim.x * blockDim.x) {
+        const unsigned row = p / nz, z = p - row * nz, x = row / ny, y = row - x * ny;
+        const unsigned px = x + 1 == (unsigned)nx ? p - (nx - 1) * ny * nz : p + ny * nz;
+        const unsigned py = y + 1 == (unsigned)ny ? p - (ny - 1) * nz : p + nz;
+        const unsigned pz = z + 1 == (unsigned)nz ? p - (nz - 1) : p + 1;
 #pragma unroll
         for (int n1 = 0; n1 < 3; ++n1) {
-            const double c = pos[n1 * V + p];
-            g[(n1 * 3 + 0) * V + p] = (pos[n1 * V + px] - c) / vs[n1];
-            g[(n1 * 3 + 1) * V + p] = (pos[n1 * V + py] - c) / vs[n1];
-            g[(n1 * 3 + 2) * V + p] = (pos[n1 * V + pz] - c) / vs[n1];
+            const double *f = pos + (size_t)n1 * V;
+            double *o = g + (size_t)n1 * 3 * V + p;
+            const double c = f[p];
+            s[n1] += c;
+            o[0] = EXACT ? (f[px] - c) * vs[n1] : (f[px] - c) / vs[n1];
+            o[V] = EXACT ? (f[py] - c) * vs[n1] : (f[py] - c) / vs[n1];
+            o[2 * (size_t)V] = EXACT ? (f[pz] - c) * vs[n1] : (f[pz] - c) / vs[n1];
         }
     }
+    add_sums(s, red);
 }
 
 template <int N>
@@ -642,21 +660,24 @@ __global__ void corner2d_kernel(const double *pos, int nx, int ny, double vol, d
 }
 
 // topology_correction_2D.cpp:209-246: periodic forward differences, g[(n1*2+n2)][p] =
-// (pos_n1(p + e_n2) - pos_n1(p)) / vs[n1]
+// (pos_n1(p + e_n2) - pos_n1(p)) / vs[n1], and the sums of the positions into red
 __global__ void gradient2d_kernel(const double *pos, int nx, int ny, double v0, double v1,
-                                  double *g) {
-    const long V = (long)nx * ny;
-    for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < V;
-         p += (long)gridDim.x * blockDim.x) {
-        const int x = (int)(p / ny), y = (int)(p % ny);
-        const long px = (long)(x + 1 > nx - 1 ? x + 1 - nx : x + 1) * ny + y;
-        const long py = (long)x * ny + (y + 1 > ny - 1 ? y + 1 - ny : y + 1);
+                                  double *g, Red *red) {
+    const int V = nx * ny;
+    double s[2] = {0.0, 0.0};
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < V; p += gridDim.x * blockDim.x) {
+        const int x = p / ny, y = p - x * ny;
+        const int px = x + 1 == nx ? y : p + ny;
+        const int py = y + 1 == ny ? x * ny : p + 1;
         const double c0 = pos[p], c1 = pos[V + p];
-        g[0 * V + p] = (pos[px] - c0) / v0;
-        g[1 * V + p] = (pos[py] - c0) / v0;
+        s[0] += c0;
+        s[1] += c1;
+        g[p] = (pos[px] - c0) / v0;
+        g[V + p] = (pos[py] - c0) / v0;
         g[2 * V + p] = (pos[V + px] - c1) / v1;
         g[3 * V + p] = (pos[V + py] - c1) / v1;
     }
+    add_sums(s, red);
 }
 
 // backward-difference divergence (periodic) of each component's 2D gradient row
@@ -672,17 +693,6 @@ __global__ void divergence2d_kernel(const double *g, int nx, int ny, double *div
             const double *gx = g + (n * 2 + 0) * V, *gy = g + (n * 2 + 1) * V;
             div[n * V + p] = (gx[p] - gx[px]) + (gy[p] - gy[py]);
         }
-    }
-}
-
-__global__ void sum_kernel(const double *pos, long V, int N, Red *red) {
-    double s[3] = {0.0, 0.0, 0.0};
-    for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < V;
-         p += (long)gridDim.x * blockDim.x)
-        for (int n = 0; n < N; ++n) s[n] += pos[n * V + p];
-    for (int n = 0; n < N; ++n) {
-        double v = warp_sum(s[n]);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&red->sum[n], v);
     }
 }
 
@@ -942,6 +952,12 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
     const int nx = w.nx, ny = w.ny, nz = w.nz;
     const long V = w.V, cells = w.cells;
     const double vol = 1.0 / (vs[0] * vs[1] * vs[2]);
+    // powers of two, with reciprocals that are too
+    bool exact = true;
+    for (int n = 0; n < 3; ++n) {
+        int e = 0;
+        exact = exact && std::frexp(vs[n], &e) == 0.5 && std::isfinite(1.0 / vs[n]);
+    }
     TopologyResult res{};
     BINDER_CUDA(cudaMemsetAsync(w.flags.p, 0, sizeof(unsigned), s));
 
@@ -970,8 +986,14 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
         Red c = corners();
         int inner = 0;
         while ((c.below > 0 || c.above > 0) && inner < max_inner) {
-            count_launch(), gradient_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, nx, ny, nz, vs[0], vs[1], vs[2],
-                                                        w.grad.p);
+            // (the sums of the positions onto the zeros that corners() left)
+            count_launch();
+            if (exact)
+                gradient_kernel<true><<<grid_for(V), 256, 0, s>>>(
+                    w.pos.p, nx, ny, nz, 1.0 / vs[0], 1.0 / vs[1], 1.0 / vs[2], w.grad.p, w.red.p);
+            else
+                gradient_kernel<false><<<grid_for(V), 256, 0, s>>>(
+                    w.pos.p, nx, ny, nz, vs[0], vs[1], vs[2], w.grad.p, w.red.p);
             LimiterArgs la{};
             la.mask = w.mask.p;
             la.g = w.grad.p;
@@ -984,8 +1006,6 @@ TopologyResult TopologyWorkspace::run(double e1, double e2, int max_outer, int m
             la.flags = w.flags.p;
             launch_limiter(la, (long)(c.below + c.above), s);
             BINDER_CUDA(cudaGetLastError());
-            // the mean position, from the zeros that corners() left
-            count_launch(), sum_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, V, 3, w.red.p);
             count_launch(), divergence_kernel<<<grid_for(V), 256, 0, s>>>(w.grad.p, nx, ny, nz, w.div.p);
             BINDER_CUDA(cudaGetLastError());
 
@@ -1064,8 +1084,9 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
         Red c = corners();
         int inner = 0;
         while ((c.below > 0 || c.above > 0) && inner < max_inner) {
+            // (the sums of the positions onto the zeros that corners() left)
             count_launch(), gradient2d_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, nx, ny, vs[0],
-                                                                          vs[1], w.grad.p);
+                                                                          vs[1], w.grad.p, w.red.p);
             LimiterArgs la{};
             la.mask = w.mask.p;
             la.g = w.grad.p;
@@ -1074,8 +1095,6 @@ TopologyResult TopologyWorkspace::run2d(double e1, double e2, int max_outer, int
             la.flags = w.flags.p;
             launch_limiter(la, (long)(c.below + c.above), s);
             BINDER_CUDA(cudaGetLastError());
-            // the mean position, from the zeros that corners() left
-            count_launch(), sum_kernel<<<grid_for(V), 256, 0, s>>>(w.pos.p, V, 2, w.red.p);
             count_launch(), divergence2d_kernel<<<grid_for(V), 256, 0, s>>>(w.grad.p, nx, ny,
                                                                             w.div.p);
             BINDER_CUDA(cudaGetLastError());

@@ -46,3 +46,13 @@ def test_hartley_forms(core, oracle, shape):
     want, outer = oracle.topology3d(f, 0.05, 20.0, 1, 1, VS, shape)
     assert tc.last_stats["outer_iterations"] == outer
     np.testing.assert_allclose(got.ravel(), want, rtol=0, atol=1e-9)
+
+
+@pytest.mark.parametrize("vs", [(2.0, 0.5, 1.0), (2.0, 3.0, 1.0)])
+def test_voxel_sizes(core, oracle, vs):
+    """Voxel sizes that are all powers of two (no division) and not."""
+    shape = (9, 16, 31)
+    f = field(shape, 0.8, 1.0, 5)
+    got = core.topology_correction_3D().correct_topology(f, 0.05, 20.0, 1, 2, 1, vs, *shape)
+    want, _ = oracle.topology3d(f, 0.05, 20.0, 1, 2, vs, shape)
+    np.testing.assert_allclose(got.ravel(), want, rtol=0, atol=1e-9)
