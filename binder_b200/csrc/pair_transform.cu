@@ -26,8 +26,8 @@
 // What bounds it (160x192x160, per tile of 8 us): the single issuing thread of the MMAs (7.2 us)
 // and the epilogue warps (7.5 us), neither HBM (a pass moves 118 MB, 18 us of its 65 us) nor the
 // matrix copies (without them 2% less).  Measured against the six per-axis passes on three streams:
-// M-step 0.294 -> 0.198 ms at 160x192x160, 58 -> 46 us at 96^3, 51 -> 28 us at 64^3; the passes of
-// a sweep of 32 chains at 96^3 1.67 -> 0.83 ms.
+// M-step 0.294 -> 0.195 ms at 160x192x160, 58 -> 38 us at 96^3, 51 -> 27 us at 64^3; the passes of
+// a sweep of 32 chains at 96^3 1.67 -> 0.82 ms.
 // Tried on the way: one CTA per tile with the same warps loading and storing 0.296 ms; the steps of
 // the MMA warp one K chunk of 16 long 0.264 ms (its waits and commits took as long as its MMAs);
 // one group of load warps instead of two 0.240 ms; 32 accumulator columns per TMEM load instead of
