@@ -46,7 +46,6 @@ struct HArgs {
     HartleyArgs a;
     const double *cs, *sn;
     int n, cols, tiles;  // tiles: 8-row tiles of the halves
-    long nlines;
 };
 
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {

@@ -168,37 +168,48 @@ __global__ void jacobian2d_kernel(const double *f, long ps, long cs, int nx, int
 // topology_correction_3D.cpp:488-607: the 8 vertex Jacobians of every cell, in the vertex order
 // 000, 100, 010, 001, 011, 101, 110, 111, each from the three cell edges through its vertex.
 // Positions are SoA [3][V].  The limiter asks only which of them lie outside [e1, e2]: bit c of
-// mask[cell] (storing the eight values moved 64 B per cell and took twice as long).
+// mask[cell] (storing the eight values moved 64 B per cell and took twice as long).  The two corners of
+// an edge share its difference, and V <= 2^24 keeps the indices in 32 bits.  Bound by the FP64 pipe.
+// 160x192x160: 110 us with an edge per corner and 64-bit indices, 88 us so.
 __global__ void corner_kernel(const double *pos, int nx, int ny, int nz, double vol, double e1,
                               double e2, uint8_t *mask, Red *red) {
-    const long V = (long)nx * ny * nz;
-    const long cy = ny - 1, cz = nz - 1;
-    const long cells = (long)(nx - 1) * cy * cz;
-    const int vert[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1},
-                            {0, 1, 1}, {1, 0, 1}, {1, 1, 0}, {1, 1, 1}};
+    const unsigned V = (unsigned)nx * ny * nz, cy = ny - 1, cz = nz - 1;
+    const unsigned cells = (unsigned)(nx - 1) * cy * cz;
+    constexpr int vert[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1},
+                                {0, 1, 1}, {1, 0, 1}, {1, 1, 0}, {1, 1, 1}};
     unsigned long long lb = 0, la = 0;
-    for (long cell = (long)blockIdx.x * blockDim.x + threadIdx.x; cell < cells;
-         cell += (long)gridDim.x * blockDim.x) {
-        const int x = (int)(cell / (cy * cz)), y = (int)((cell / cz) % cy), z = (int)(cell % cz);
+    for (unsigned cell = blockIdx.x * blockDim.x + threadIdx.x; cell < cells;
+         cell += gridDim.x * blockDim.x) {
+        const unsigned row = cell / cz, z = cell - row * cz, x = row / cy, y = row - x * cy;
+        const double *node = pos + ((size_t)(x * ny + y) * nz + z);
+        // the cell's edges along each axis, [the two other coordinates][component], far end minus
+        // near end: two corners share each
+        double ex[4][3], ey[4][3], ez[4][3];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            double p[2][2][2];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < 2; ++b)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+                        p[a][b][c] = node[(size_t)m * V + (unsigned)((a * ny + b) * nz + c)];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    ex[2 * a + b][m] = p[1][a][b] - p[0][a][b];
+                    ey[2 * a + b][m] = p[a][1][b] - p[a][0][b];
+                    ez[2 * a + b][m] = p[a][b][1] - p[a][b][0];
+                }
+        }
         unsigned bits = 0;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-            const int vx = vert[c][0], vy = vert[c][1], vz = vert[c][2];
-            const long pw = ((long)(x + vx) * ny + (y + vy)) * nz + (z + vz);
-            const long pxn = ((long)(x + 1 - vx) * ny + (y + vy)) * nz + (z + vz);
-            const long pyn = ((long)(x + vx) * ny + (y + 1 - vy)) * nz + (z + vz);
-            const long pzn = ((long)(x + vx) * ny + (y + vy)) * nz + (z + 1 - vz);
-            double col[3][3];
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                const double w = pos[m * V + pw];
-                const double a = pos[m * V + pxn], b = pos[m * V + pyn], d = pos[m * V + pzn];
-                col[0][m] = vx ? w - a : a - w;
-                col[1][m] = vy ? w - b : b - w;
-                col[2][m] = vz ? w - d : d - w;
-            }
-            double j = det3(col[0][0], col[1][0], col[2][0], col[0][1], col[1][1], col[2][1],
-                            col[0][2], col[1][2], col[2][2]);
+            const double *u = ex[2 * vert[c][1] + vert[c][2]], *v = ey[2 * vert[c][0] + vert[c][2]],
+                         *w = ez[2 * vert[c][0] + vert[c][1]];
+            double j = det3(u[0], v[0], w[0], u[1], v[1], w[1], u[2], v[2], w[2]);
             j *= vol;
             lb += j < e1;
             la += j > e2;
