@@ -43,41 +43,51 @@ struct Red {
     int pad;
 };
 
-// BINDER/src/cpu/utils.cpp:100-345.  Element (p, m) of the field is f[p*ps + m*cs].
+// BINDER/src/cpu/utils.cpp:100-345.  Element (p, m) of the field is f[p*ps + m*cs].  Four corners
+// share each difference; bound by the FP64 pipe.  160x192x160: 164 us with the differences taken
+// per corner, 97 us so.
 __global__ void jacobian_kernel(const double *f, long ps, long cs, int nx, int ny, int nz,
                                 double vol, double *J, double e1, double e2, Red *red) {
     const long V = (long)nx * ny * nz;
     const long yz = (long)ny * nz;
     // corner order of the reference: fff, bff, fbf, ffb, bbf, bfb, fbb, bbb
-    const int dir[8][3] = {{1, 1, 1},  {-1, 1, 1},  {1, -1, 1},  {1, 1, -1},
+    constexpr int dir[8][3] = {{1, 1, 1},  {-1, 1, 1},  {1, -1, 1},  {1, 1, -1},
                            {-1, -1, 1}, {-1, 1, -1}, {1, -1, -1}, {-1, -1, -1}};
     double lmin = 1e300, lmax = -1e300;
     unsigned long long lb = 0, la = 0, ln = 0;
     for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < V;
          p += (long)gridDim.x * blockDim.x) {
-        const int x = (int)(p / yz), y = (int)((p / nz) % ny), z = (int)(p % nz);
-        double w0[3];
-        for (int m = 0; m < 3; ++m) w0[m] = f[p * ps + m * cs];
+        int x, y, z;
+        if (V <= 0xffffffffL) {  // 32-bit divisions
+            const unsigned q = (unsigned)p, row = q / (unsigned)nz;
+            z = (int)(q - row * nz);
+            x = (int)(row / (unsigned)ny);
+            y = (int)(row - (unsigned)x * ny);
+        } else {
+            x = (int)(p / yz), y = (int)((p / nz) % ny), z = (int)(p % nz);
+        }
+        // the differences to the next (0) and from the previous (1) point along each axis, where
+        // there is one (the point itself stands in where there is none)
+        const bool ok[3][2] = {{x < nx - 1, x > 0}, {y < ny - 1, y > 0}, {z < nz - 1, z > 0}};
+        const long step[3] = {yz, nz, 1};
+        double d[3][2][3];  // [axis][side][component]
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const double w0 = f[p * ps + m * cs];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                d[a][0][m] = f[(ok[a][0] ? p + step[a] : p) * ps + m * cs] - w0;
+                d[a][1][m] = w0 - f[(ok[a][1] ? p - step[a] : p) * ps + m * cs];
+            }
+        }
         double tot = 0.0;
         int valid = 0;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-            const int sx = dir[c][0], sy = dir[c][1], sz = dir[c][2];
-            if ((sx > 0 && x >= nx - 1) || (sx < 0 && x <= 0)) continue;
-            if ((sy > 0 && y >= ny - 1) || (sy < 0 && y <= 0)) continue;
-            if ((sz > 0 && z >= nz - 1) || (sz < 0 && z <= 0)) continue;
-            const long qx = p + sx * yz, qy = p + sy * nz, qz = p + sz;
-            double col[3][3];  // [axis][component]
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                const double ax = f[qx * ps + m * cs], ay = f[qy * ps + m * cs],
-                             az = f[qz * ps + m * cs];
-                col[0][m] = sx > 0 ? ax - w0[m] : w0[m] - ax;
-                col[1][m] = sy > 0 ? ay - w0[m] : w0[m] - ay;
-                col[2][m] = sz > 0 ? az - w0[m] : w0[m] - az;
-            }
-            const double jc = det3(col[0][0], col[1][0], col[2][0], col[0][1], col[1][1], col[2][1],
-                                   col[0][2], col[1][2], col[2][2]) * vol;
+            const int sx = dir[c][0] < 0, sy = dir[c][1] < 0, sz = dir[c][2] < 0;
+            if (!(ok[0][sx] && ok[1][sy] && ok[2][sz])) continue;
+            const double *u = d[0][sx], *v = d[1][sy], *w = d[2][sz];
+            const double jc = det3(u[0], v[0], w[0], u[1], v[1], w[1], u[2], v[2], w[2]) * vol;
             tot += jc;
             valid++;
         }
