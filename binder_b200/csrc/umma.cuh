@@ -74,8 +74,11 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // ---- TMEM ------------------------------------------------------------------------------------
+// Whole warps only: the .aligned forms are undefined in a warp whose lanes have parted, as they do
+// around the stores of a tile's last, partial rows, so each wrapper brings the warp together first.
 // one warp: allocate ncols (power of two >= 32) columns, address written to *holder
 __device__ __forceinline__ void tmem_alloc(uint32_t *holder, uint32_t ncols) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(holder)),
                  "r"(ncols)
@@ -83,6 +86,7 @@ __device__ __forceinline__ void tmem_alloc(uint32_t *holder, uint32_t ncols) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                  : "memory");
 }
@@ -90,6 +94,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 // 32 consecutive FP32 columns of this thread's TMEM lane (warp w reads lanes 32w..32w+31)
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     uint32_t r[32];
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
         "%11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, "
@@ -109,6 +114,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 // 16 consecutive FP32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
         "%11, %12, %13, %14, %15}, [%16];"
