@@ -207,6 +207,15 @@ __device__ __forceinline__ void col_add2(float *__restrict__ col, int ka, int kb
     col[ka * TPB] = na;
     col[kb * TPB] = nb;
 }
+// A voxel whose total weight S is so small that scale / S, or 1 / S, is past FP32's range: S, its
+// moments and the column masses of bins lo .. hi are multiplied by 2^64, which no ratio of them
+// feels.  (A mass times an infinite scale / S is an infinity, which the conversion to fixed point
+// makes 2^32 - 1.)
+constexpr float kLift = 18446744073709551616.0f;  // 2^64
+template <int TPB>
+__device__ __forceinline__ void col_lift(float *__restrict__ col, int lo, int hi) {
+    for (int k = lo; k <= hi; ++k) col[k * TPB] *= kLift;
+}
 template <int TPB>
 __device__ __forceinline__ void col_add2(__half *__restrict__ col, int ka, int kb, float2 w) {
     const __half2 h = __float22half2_rn(w);
@@ -598,8 +607,15 @@ __global__ void __launch_bounds__(TPB, 1) estep_filter_col_kernel(const EStepArg
             }
         }
         const bool ok = S > 0.0f;
-        const float inv = ok ? 1.0f / S : 0.0f;
-        const float invs = inv * a.hscale;
+        float inv = ok ? 1.0f / S : 0.0f, invs = inv * a.hscale;
+        // four channels of starting theta entries of 1e-8 come here
+        if (ok && isinf(invs)) {
+#pragma unroll
+            for (int m = 0; m < MC; ++m) col_lift<TPB>(my + (size_t)m * K4 * TPB, lo[m], hi[m]);
+            Sx *= kLift, Sy *= kLift, Sz *= kLift;
+            inv = 1.0f / (S * kLift);
+            invs = inv * a.hscale;
+        }
 #pragma unroll
         for (int m = 0; m < MC; ++m) {
             unsigned *hcol = hs + (size_t)m * K * LP + um[m];
