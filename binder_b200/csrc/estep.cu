@@ -401,6 +401,10 @@ __device__ __forceinline__ void merge_cta(const EStepArgs &a, const unsigned *hs
 // histogram stay FP32 / fixed point; only the per-voxel bin sums are rounded to FP16.
 constexpr float kHalfColScale = 4096.0f;
 constexpr double kLnHalfColScale = 8.317766166719343;  // ln 4096
+// The FP32 columns of the MI likelihood stage theta times 2^32, an exact factor that cancels in every
+// ratio to S: with theta as it is, a total weight S below about 2.5e-32 makes hscale / S infinite and
+// the fixed-point masses 2^32 - 1.
+constexpr float kThetaScale = 4294967296.0f;
 
 template <int TPB, int DIM, bool LOGT, bool HC = false>
 __global__ void __launch_bounds__(TPB, HC ? 3 : (TPB > kFastThreads ? 1 : 2))
@@ -420,7 +424,7 @@ __global__ void __launch_bounds__(TPB, HC ? 3 : (TPB > kFastThreads ? 1 : 2))
     __shared__ double red[32];
     if (LOGT)
         for (int l = threadIdx.x; l < L; l += TPB) cmx[l] = a.colmax[l];
-    const float tscale = HC ? kHalfColScale : 1.0f;
+    constexpr float tscale = HC ? kHalfColScale : LOGT ? 1.0f : kThetaScale;
 #pragma unroll 4
     for (int q = threadIdx.x; q < KL; q += TPB) {
         const int k = q / L, l = q - k * L;
@@ -458,7 +462,8 @@ __global__ void __launch_bounds__(TPB, HC ? 3 : (TPB > kFastThreads ? 1 : 2))
                                       kmax, mlog);
         else
             em_accumulate<TPB, Q>(thT + ui * KP, my, pk, bx, by, bz, S, Sx, Sy, Sz, kmin, kmax);
-        const bool ok = S > 0.0f;
+        const float S1 = HC || LOGT ? S : S * (1.0f / kThetaScale);  // without the staged scale
+        const bool ok = S1 > 0.0f;
         const float inv = ok ? 1.0f / S : 0.0f;
         const float invs = inv * a.hscale;
         unsigned *hcol = hs + ui;  // hcol[k * LP]
@@ -481,7 +486,7 @@ __global__ void __launch_bounds__(TPB, HC ? 3 : (TPB > kFastThreads ? 1 : 2))
             ++deg;
             continue;
         }
-        mll -= (double)logf(S);  // FP32 log, FP64 accumulation
+        mll -= (double)logf(S1);  // FP32 log, FP64 accumulation
         if (HC) mll += kLnHalfColScale;
         if (LOGT) mll -= (double)mlog * 0.6931471805599453 + (double)cmx[ui];
         vp.store_r(a, i, V, fx + Sx * inv, fy + Sy * inv, fz + Sz * inv);

@@ -6,7 +6,9 @@ entries adds three roundings of 6e-8)."""
 import numpy as np
 import pytest
 
+from test_gpu_edge_cases import one_iteration
 from test_gpu_mi_filter import filter_case, new_filter_reg, oracle_iteration
+from test_gpu_parity import make_case
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +40,14 @@ def test_filter_channels(core, oracle, M, floor):
     np.testing.assert_allclose(reg.get_final_locations_as_numpy_array().ravel(), final, rtol=0,
                                atol=2e-4)
     assert reg.iteration_stats()[0][0] == pytest.approx(mll, rel=1e-6)
+
+
+@pytest.mark.parametrize("shape", [(12, 10, 9), (97, 97, 97)])
+def test_one_channel(core, oracle, shape):
+    """The 256- and the 768-thread form."""
+    c = make_case(shape=shape, K=8, L=6, seed=7)
+    V = int(np.prod(shape))
+    th, v, u = floored(1, 8, 6, 1e-33, c["v"].reshape(V, 1), c["u"].reshape(V, 1))
+    c["theta"] = th[0]
+    c["v"], c["u"] = v.reshape(c["v"].shape), u.reshape(c["u"].shape)
+    one_iteration(core, oracle, c)
