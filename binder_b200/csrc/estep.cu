@@ -522,8 +522,19 @@ __device__ __forceinline__ void merge_mll(const double *mpart, DevState *st, dou
 // weight of a neighbour is its spline weight times prod_m theta[m][k_m][u_m]; it is added to every
 // channel's column, and the columns are flushed once per voxel as hist[m][k][u_m] += col / S in
 // fixed point.  Against two passes with one shared FP32 atomic (a compare-and-swap loop) per
-// neighbour and channel: 349 -> 79 us per launch at 64^3 with two channels of 48 bins.
+// neighbour and channel: 349 -> 80 us per launch at 64^3 with two channels of 48 bins.
 // Bound by the same issue and latency as the MI kernel, with as many warps as the columns leave.
+//
+// A cell of the CTA's histogram is 32 bits that wrap, their carries going to the 64-bit sums at once,
+// so the scale is 2^27 whatever the volume: a posterior is kept to 3.7e-9.  At a scale for which a
+// CTA's voxels fit in 32 bits (2.4e6 at 64^3, 1.3e5 at 160x192x160) the small masses, which are all
+// that a rare pair of bins has, are dropped.  Error of theta's cells against 64 bits after an
+// iteration from a registered state, mean / worst: 4e-8 / 6e-7 at 64^3 and 6e-8 / 3e-6 at
+// 160x192x160, against 1e-6 / 6e-5 and 1e-4 / 1e-2 at those scales, and 2e-7 / 2e-6 and 8e-7 / 4e-5
+// for FP32 sums.  The carries cost 2 to 5 % of a launch; testing each of the four old values by
+// itself, 6 to 13 %.
+constexpr float kFilterScale = 134217728.0f;
+constexpr unsigned kFilterFull = 0xf7000000u;  // 2^32 - 2^27 (1 + 1/8)
 template <int DIM, int MC, int TPB>
 __global__ void __launch_bounds__(TPB, 1) estep_filter_col_kernel(const EStepArgs a) {
     constexpr int Q = DIM == 3 ? 4 : 1;
@@ -624,17 +635,23 @@ __global__ void __launch_bounds__(TPB, 1) estep_filter_col_kernel(const EStepArg
 #pragma unroll
         for (int m = 0; m < MC; ++m) {
             unsigned *hcol = hs + (size_t)m * K * LP + um[m];
+            unsigned long long *hg = a.hfix + (size_t)m * KL + um[m];
             float *col = my + (size_t)m * K4 * TPB;
             for (int k = lo[m] & ~3; k <= hi[m]; k += 4) {
-                float v[4];
+                unsigned x[4], was[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) v[e] = col[(k + e) * TPB];
+                for (int e = 0; e < 4; ++e) x[e] = __float2uint_rn(col[(k + e) * TPB] * invs);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    if (ok && v[e] != 0.0f)
-                        atomicAdd(&hcol[(k + e) * LP], __float2uint_rn(v[e] * invs));
+                    was[e] = 0u;
+                    if (x[e]) was[e] = atomicAdd(&hcol[(k + e) * LP], x[e]);
                     col[(k + e) * TPB] = 0.0f;
                 }
+                // near enough to 2^32 for a posterior of 1 (and its roundings) to pass it
+                if (__vimax3_u32(__vimax3_u32(was[0], was[1], was[2]), was[3], 0u) >= kFilterFull)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (was[e] > ~x[e]) atomicAdd(&hg[(k + e) * L], 1ull << 32);
             }
         }
         if (!ok) {
@@ -2006,6 +2023,7 @@ void launch_estep(const EStepArgs &args, bool sample, int grid, cudaStream_t s, 
     sc = sc < 1.0 ? 1.0 : (sc > 1073741824.0 ? 1073741824.0 : sc);
     float fsc = (float)sc;
     if ((double)fsc > sc) fsc = std::nextafter(fsc, 0.0f);  // round down into FP32
+    if (a.filter && !sample && ftpb != kFilterPasses) fsc = kFilterScale;  // cells that carry
     a.hscale = fsc;
     a.hinv = 1.0 / (double)fsc;
     BINDER_CHECK(a.dim == 2 || a.dim == 3, "dimension must be 2 or 3");
