@@ -45,7 +45,7 @@ double spline_sigma2(int order) {
 }
 
 // `p` (freed first) becomes n slots of `slot` floats, fewer where the memory for them is not there,
-// one at least; returns their number.  The ring lives for one sampler call.
+// one at least; returns their number.
 int alloc_ring(float *&p, long slot, int n, cudaStream_t s) {
     dfree(p, s);
     for (;; n /= 2) {
@@ -58,6 +58,20 @@ int alloc_ring(float *&p, long slot, int n, cudaStream_t s) {
         }
     }
 }
+
+// Gives a sampler call's ring back to the pool of stream `own` once the sweeps on `work` are done,
+// before the moments' staging asks for as much memory, or when the call ends early.
+struct RingGuard {
+    float *&p;
+    cudaStream_t work, own;
+    ~RingGuard() { release(); }
+    void release() {
+        if (!p) return;
+        cudaStreamSynchronize(work);
+        dfree(p, own);
+        cudaStreamSynchronize(own);  // the staging comes from `work`
+    }
+};
 
 struct Graph {
     cudaGraph_t g = nullptr;
@@ -975,6 +989,7 @@ void Registration::sampler(uint64_t seed, int N_b, int N_s, int sample_gamma,
     const int total = N_b + N_s;
     const long slot = (long)V_ * N_;
     int R = sampler_ring(mstep_, 1, total, sample_posteriors, sample_transformation_parameters);
+    RingGuard ring{ring_, stream_, own_stream_};
     if (total > 0 && sample_transformation_parameters) {
         mstep_.prepare_sampling(own_stream_);
         if (R > 1) R = alloc_ring(ring_, slot, R, own_stream_);
@@ -1040,6 +1055,7 @@ void Registration::sampler(uint64_t seed, int N_b, int N_s, int sample_gamma,
     }
     DevState h{};
     BINDER_CUDA(cudaMemcpyAsync(&h, st_, sizeof(DevState), cudaMemcpyDeviceToHost, stream_));
+    ring.release();
     // moments rearranged to AoS on the device, then one transfer each
     double *mean_aos = dalloc<double>((size_t)V_ * N_, stream_);
     double *cov_aos = dalloc<double>((size_t)V_ * N_ * N_, stream_);
@@ -1051,7 +1067,6 @@ void Registration::sampler(uint64_t seed, int N_b, int N_s, int sample_gamma,
     dfree(mean_aos, stream_);
     dfree(cov_aos, stream_);
     BINDER_CUDA(cudaStreamSynchronize(stream_));
-    dfree(ring_, own_stream_);
     for (int n = 0; n < 3; ++n) gamma0_[n] = h.gamma[n];  // the prior keeps sampled gammas
 }
 
@@ -1109,6 +1124,7 @@ void Registration::sampler_chains(uint64_t seed, int chains, int N_b, int N_s, i
     }
     const int total = N_b + N_s;
     const long slot = (long)(VN * C);
+    RingGuard ring{cb_->ring, stream_, so};
     const int R = alloc_ring(cb_->ring, slot,
                              sampler_ring(cb_->mstep, C, total, sample_posteriors,
                                           sample_transformation_parameters), so);
@@ -1179,6 +1195,7 @@ void Registration::sampler_chains(uint64_t seed, int chains, int N_b, int N_s, i
         if (verbose())
             std::printf("sampler: %d chains x %d sweeps in %.3f ms\n", C, total, ms);
     }
+    ring.release();
     // moments: per chain rearranged to AoS on the device and read back in one copy each, and / or
     // pooled over the chains
     const double scale = 1.0 / (double)(N_s - 1);
@@ -1213,7 +1230,6 @@ void Registration::sampler_chains(uint64_t seed, int chains, int N_b, int N_s, i
     dfree(mstage, stream_);
     dfree(cstage, stream_);
     BINDER_CUDA(cudaStreamSynchronize(stream_));
-    dfree(b.ring, so);
 }
 
 double Registration::profile_stage(int stage, int n) {
