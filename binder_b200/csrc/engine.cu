@@ -1305,6 +1305,9 @@ void Registration::reset() {
         BINDER_CUDA(cudaMemcpyAsync(theta_, theta0_, sizeof(float) * M_ * K_ * L_,
                                     cudaMemcpyDeviceToDevice, stream_));
         BINDER_CUDA(cudaMemsetAsync(hist_, 0, sizeof(float) * M_ * K_ * L_, stream_));
+        if (hfix_)  // the sums of an E-step whose update did not come
+            BINDER_CUDA(cudaMemsetAsync(hfix_, 0, sizeof(unsigned long long) * M_ * K_ * L_,
+                                        stream_));
         BINDER_CUDA(cudaMemsetAsync(hcnt_, 0, sizeof(unsigned) * M_ * K_ * L_, stream_));
     }
     if (lk_ == 1) {

@@ -2011,6 +2011,10 @@ void launch_estep(const EStepArgs &args, bool sample, int grid, cudaStream_t s, 
                                           : filter_smem(a.K, a.L, a.M, sample))
                                    : estep_smem(sample, a.K, a.L, a.logt != 0, a.halfcol != 0,
                                                 ftpb);
+    const bool single_pass = !sample && !a.ssdf &&
+                             (a.filter ? ftpb != kFilterPasses : a.K <= kSmallK);
+    BINDER_CHECK(!single_pass || (a.hfix && a.mpart),
+                 "the single-pass EM kernels need the buffers of their merge");
     // the order-independent merge of the single-pass EM kernel keeps one partial per CTA
     if (a.hfix && grid > kMaxEmCtas) grid = kMaxEmCtas;
     // fixed-point scale of the EM histogram: the largest scale (at most 2^30, exact in FP32) for
@@ -2023,7 +2027,7 @@ void launch_estep(const EStepArgs &args, bool sample, int grid, cudaStream_t s, 
     sc = sc < 1.0 ? 1.0 : (sc > 1073741824.0 ? 1073741824.0 : sc);
     float fsc = (float)sc;
     if ((double)fsc > sc) fsc = std::nextafter(fsc, 0.0f);  // round down into FP32
-    if (a.filter && !sample && ftpb != kFilterPasses) fsc = kFilterScale;  // cells that carry
+    if (a.filter && single_pass) fsc = kFilterScale;  // cells that carry
     a.hscale = fsc;
     a.hinv = 1.0 / (double)fsc;
     BINDER_CHECK(a.dim == 2 || a.dim == 3, "dimension must be 2 or 3");

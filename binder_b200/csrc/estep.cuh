@@ -21,9 +21,10 @@ struct EStepArgs {
     const uint8_t *vpad;  // moving-image bins, zero-padded [nxn+2P][nyn+2P][zp bytes]
     const float *theta;   // [K*L]
     float *hist;          // EM: soft joint histogram [K*L] (accumulated)
-    // the single-pass EM kernel's order-independent merge (both null: FP32 atomics instead): 64-bit
-    // fixed-point sums [K*L], and one log-likelihood partial per CTA [kMaxEmCtas] followed by the
-    // sums' scale and the number of CTAs; the likelihood update that follows reads and clears them
+    // the single-pass EM kernels' order-independent merge, which they need (the others add to hist
+    // and st->mll; both null is fine there): 64-bit fixed-point sums [M*K*L], and one log-likelihood
+    // partial per CTA [kMaxEmCtas] followed by the sums' scale and the number of CTAs; the likelihood
+    // update that follows reads them and clears the sums
     unsigned long long *hfix;
     double *mpart;
     unsigned *hcnt;       // Gibbs: joint counts [K*L] (accumulated)
