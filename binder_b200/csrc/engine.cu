@@ -292,6 +292,8 @@ void MStep::enqueue(const float *r, float *d, const float *xpos, const float *D,
     a.nz = nz;
     const int ncomp = nz == 1 ? 2 : 3;
     a.dims = ncomp;
+    // an MMA has at most 256 columns, and a slab of the FP32 passes 256 rows
+    BINDER_CHECK(nx <= 256 && ny <= 256 && nz <= 256, "transform axis length must be in [1, 256]");
     if (fused2d) {
         a.comp0 = 0;
         a.xpos = xpos;
