@@ -320,7 +320,8 @@ void MStep::enqueue(const float *r, float *d, const float *xpos, const float *D,
     }
     BINDER_CHECK(ring_n <= 1 || (paired() && nz > 1),
                  "a ring of positions needs the paired passes");
-    // BF16 operands and axes of at most 256: two passes per launch, all components in one launch
+    // BF16 operands and planes that fit shared memory (pair_supported: with the split, 224 x 224 and
+    // most smaller ones, not 128 x 256 or 256 x 256): two passes per launch, all components in one
     if (paired()) {
         a.chain_comps = chains > 1 ? ncomp : 0;
         run_pairs(a, ncomp * chains, planes, s, r, d, xpos);

@@ -13,7 +13,9 @@ enum PairKind : int {
 };
 
 // Whether the pair kernels take an nx x ny x nz volume (nz == 1: an image, kPairSpectral only):
-// BF16 operands, every axis at most 256 long (the MMA's N) and the tiles within shared memory.
+// BF16 operands, every axis at most 256 long (the MMA's N) and the tiles within shared memory.  With
+// the split that leaves out planes of about 241 x 81 and more, and 209 x 128 to 241 x 96 either way
+// round; their volumes take the per-axis passes.
 bool pair_supported(int nx, int ny, int nz, int planes);
 
 // One pair over `ncomp` components of a volume; `a` as for launch_axis_pass_tc (in, out, D, st,
