@@ -195,6 +195,15 @@ template <int TPB>
 __device__ __forceinline__ __half *half_slot(__half *col, int k) {
     return col + k * TPB;
 }
+// The shared address of a row of theta, for loads in an asm that is neither volatile nor clobbers
+// memory (so that they are not ordered against the columns' stores).  The value comes out of a
+// volatile asm, which stays behind the barrier that completes the table, and so do the loads.
+__device__ __forceinline__ unsigned table_address(const float *row) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(row);
+    asm volatile("" : "+r"(a)::"memory");
+    return a;
+}
+
 // masses w.x, w.y of two neighbours with bins ka, kb, added one after the other (one FP32 to FP16
 // pair conversion); the FP32 form loads both sums before either store, which halves the chain of
 // dependent shared-memory round trips (340 -> 335 us at 160x192x160; four at a time, with their
@@ -257,7 +266,7 @@ __device__ __forceinline__ void em_accumulate(const float *__restrict__ thu,
     int lo = 255, hi = 0;
     // theta's address of byte c: one dot-product instruction instead of an extraction and an add
     // (E-step 326 -> 319 us at 160x192x160); loads without memory clobber, theta is constant here
-    const unsigned tha = (unsigned)__cvta_generic_to_shared(thu);
+    const unsigned tha = table_address(thu);
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
@@ -575,7 +584,7 @@ __global__ void __launch_bounds__(TPB, 1) estep_filter_col_kernel(const EStepArg
 #pragma unroll
         for (int m = 0; m < MC; ++m) {
             um[m] = a.u[m * a.uch + i];
-            tha[m] = (unsigned)__cvta_generic_to_shared(thT + (m * L + um[m]) * KP);
+            tha[m] = table_address(thT + (m * L + um[m]) * KP);
             lo[m] = 255;
             hi[m] = 0;
         }
@@ -1322,7 +1331,7 @@ __global__ void __launch_bounds__(kEThreads, (SAMPLE && !LOGT) ? 3 : 2)
         const float *thc = th + ui * a.tpitch;  // theta of this voxel's bin: thc[k]
         const int L = a.L;
         // theta of node c of a packed word, its address by one dot-product instruction
-        const unsigned tha = (unsigned)__cvta_generic_to_shared(thc);
+        const unsigned tha = table_address(thc);
         auto theta_at = [&](uint32_t word, int c) {
             float t;
             asm("ld.shared.f32 %0, [%1];" : "=f"(t) : "r"(__dp4a(word, 4u << (8 * c), tha)));
