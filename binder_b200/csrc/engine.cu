@@ -218,8 +218,6 @@ void MStep::init(int x, int y, int z, cudaStream_t s, int nchains) {
     chains = nchains < 1 ? 1 : nchains;
     dct.init(x, y, z, s);
     t1 = dalloc<float>((size_t)V * 3 * chains, s);
-    t2 = dalloc<float>((size_t)V * 3 * chains, s);
-    precision = default_precision();
     // a persistent CTA's tiles span components (its cost sums could mix chains), and the fused 2D
     // M-step runs one chain
     persistent = chains == 1 && default_persistent();
@@ -228,6 +226,20 @@ void MStep::init(int x, int y, int z, cudaStream_t s, int nchains) {
         const bool off = e && e[0] == '0' && e[1] == 0;
         fused2d = chains == 1 && !off && z == 1 && x <= kM2dMaxN && y <= kM2dMaxN;
         if (fused2d) fused_cluster = mstep2d_cluster(e && e[0] == '8' && e[1] == 0);
+    }
+    set_precision(default_precision(), s);
+}
+
+void MStep::set_precision(int p, cudaStream_t s) {
+    const int before = precision;
+    precision = p;
+    if (t2 || fused2d || paired()) return;
+    try {
+        t2 = dalloc<float>((size_t)V * 3 * chains, s);
+        BINDER_CUDA(cudaStreamSynchronize(s));  // the work may be on another stream
+    } catch (...) {
+        precision = before;
+        throw;
     }
 }
 
@@ -375,6 +387,7 @@ void MStep::run_pairs(AxisArgs<float> a, int nc, int planes, cudaStream_t s, con
 // the pass sequence of one M-step for components [c0, c0 + nc) on stream s
 void MStep::run_chain(AxisArgs<float> a, int c0, int nc, cudaStream_t s, const float *r, float *d,
                   const float *xpos, bool tc, int planes) {
+    BINDER_CHECK(t2, "the per-axis passes need their scratch (MStep::set_precision)");
     a.comp0 = c0;
     const bool two_d = nz == 1;
     const bool bf16 = precision == kPrecBF16x3 || precision == kPrecBF16;
@@ -1120,7 +1133,7 @@ void Registration::sampler_chains(uint64_t seed, int chains, int N_b, int N_s, i
         cb_->mstep.init(nx_, ny_, nz_, so, C);
         BINDER_CUDA(cudaStreamSynchronize(so));
     }
-    cb_->mstep.precision = mstep_.precision;
+    cb_->mstep.set_precision(mstep_.precision, so);
     if (sample_transformation_parameters) {
         cb_->mstep.prepare_sampling(own_stream_);
         BINDER_CUDA(cudaStreamSynchronize(own_stream_));
@@ -1277,7 +1290,7 @@ double Registration::profile_stage(int stage, int n) {
 void Registration::set_precision(int p) {
     BINDER_CHECK(p >= 0 && p <= 4,
                  "precision must be 0 (FP32), 1 (3xTF32), 2 (TF32), 3 (BF16x3) or 4 (BF16)");
-    mstep_.precision = p;
+    mstep_.set_precision(p, own_stream_);
     em_graph_.clear();
 }
 
@@ -1294,7 +1307,7 @@ void Registration::set_chain(uint32_t c) {
 void PriorTransform::set_precision(int p) {
     BINDER_CHECK(p >= 0 && p <= 4,
                  "precision must be 0 (FP32), 1 (3xTF32), 2 (TF32), 3 (BF16x3) or 4 (BF16)");
-    mstep_.precision = p;
+    mstep_.set_precision(p, own_stream_);
 }
 
 void Registration::reset() {

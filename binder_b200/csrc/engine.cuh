@@ -27,7 +27,8 @@ struct MStep {
     int nx = 0, ny = 0, nz = 0;
     long V = 0;
     DctSet dct;
-    float *t1 = nullptr, *t2 = nullptr;
+    float *t1 = nullptr;
+    float *t2 = nullptr;  // the per-axis passes' other buffer; the paired and the fused ones need none
     int precision = kPrecFP32Simt;  // TransformPrecision
     // tensor-core passes: one CTA per 128-line tile with the components on their own streams, or
     // persistent (all components per launch, one CTA per SM; measured slower on B200)
@@ -48,6 +49,8 @@ struct MStep {
     float *noise = nullptr;
     // buffers from the stream-ordered pool on stream s
     void init(int nx, int ny, int nz, cudaStream_t s, int chains = 1);
+    // sets the precision and gets the scratch of its passes; not during a capture
+    void set_precision(int p, cudaStream_t s);
     void prepare_sampling(cudaStream_t s);
     void make_branches();
     void release(cudaStream_t s);
