@@ -236,6 +236,7 @@ void launch_mode_h(const HArgs &h, int ncomp, cudaStream_t s) {
 }  // namespace
 
 void HartleyMatrix::init(int n_, cudaStream_t s) {
+    release(s);  // of an earlier attempt, whose next allocation failed
     n = n_;
     rows = (n / 2 + 1 + 7) / 8 * 8;
     cols = (n / 2 + 1 + 3) / 4 * 4;
