@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(TPB, HC ? 3 : (TPB > kFastThreads ? 1 : 2))
     // and their 64-bit global sums are exact whatever order the CTAs arrive in.  The likelihood
     // update that follows on the stream converts the sums (one rounding per cell), clears them and
     // adds the CTAs' log-likelihood partials in CTA order (merged_cell, merge_mll).  Done here by
-    // the last CTA to finish, it held up the M-step by 13 us whatever the volume.
+    // the last CTA to finish, it held up the M-step by 9 us whatever the volume.
     merge_cta<TPB>(a, hs, K, LP, mll, deg, red);
 }
 

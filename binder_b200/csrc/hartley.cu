@@ -6,12 +6,12 @@
 // k = 0 .. n/2 give H[k] = C_k + S_k and H[n-k] = C_k - S_k: two products of (n/2)^2 instead of one
 // of n^2, half the operations.
 //
-// A CTA owns 32 (or 8) lines.  It folds them into shared memory (e and o, [j][32] with a pitch of 36
-// doubles, or [j][8] with 12: the four rows of a fragment are 8 banks apart), and each warp computes
-// its 8-row tiles of both products for all the lines with mma.m8n8k4 (FP64 in, FP64 FMA
-// accumulation), the matrices coming from global memory through L1.  kHartleyPoisson folds the
-// scaled coefficients straight from the accumulators -- a thread holds k and n - k of its lines --
-// and transforms again, so the spectrum is never stored.
+// A CTA folds its 32 (or 8) lines into shared memory (e and o, [j][32] with a pitch of 36 doubles, or
+// [j][8] with 12: the four rows of a fragment are 8 banks apart), and each warp computes its 8-row
+// tiles of both products for all the lines with mma.m8n8k4 (FP64 in, FP64 FMA accumulation), the
+// matrices coming from global memory through L1.  kHartleyPoisson folds the scaled coefficients
+// straight from the accumulators -- a thread holds k and n - k of its lines -- and transforms again,
+// so the spectrum is never stored.
 //
 // Bound: the FP64 pipe (0.5 n FMA per element and pass; 5.1 GFLOP per pass at 160x192x160, 0.14 ms at
 // 36 TFLOP/s).  Three components at 160x192x160, z / y / x with the Poisson scaling / y / z back:
@@ -19,13 +19,13 @@
 // matrix took 0.6 / 0.95 / 0.95 / 0.95 / 0.6 (one CTA of eight warps per SM, its staging not
 // overlapped, a division per staged element).
 //
-// A CTA owns 32 lines and has a warp for every two 8-row tiles of the halves (17 tiles at most, at
-// n = 256), so no warp idles but for an odd last tile, and two or three CTAs share an SM, one's
-// folding overlapping another's products.  Four warps with three or four tiles each took 0.21 / 0.29
+// A CTA of 32 lines has a warp for every two 8-row tiles of the halves (17 tiles at most, at n = 256),
+// so no warp idles but for an odd last tile, and two or three CTAs share an SM, one's folding
+// overlapping another's products.  Four warps with three or four tiles each took 0.21 / 0.29
 // / 0.34 / 0.29 / 0.21: 13 tiles leave three of 16 slots empty.  96 registers are what keeps three CTAs of
 // six warps (or of seven) on an SM; with 128 the passes are 10 to 15 % slower, with 80 (three CTAs
-// asked for of seven warps) 30 %.  Where 32 lines would leave SMs without a CTA, a CTA owns 8 lines
-// and has a warp per tile (two components at 128x128, y / x with the Poisson scaling / y back: 4.4 /
+// asked for of seven warps) 30 %.  Where 32 lines would leave SMs without a CTA, a CTA has 8 lines
+// and a warp per tile (two components at 128x128, y / x with the Poisson scaling / y back: 4.4 /
 // 6.8 / 4.4 us, against 14.6 / 29.0 / 14.8 with 32 lines).
 #include <cmath>
 #include <vector>

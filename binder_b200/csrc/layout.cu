@@ -132,7 +132,7 @@ __global__ void moments_to_aos_kernel(const double *mean, const double *m2, long
 //
 // Bound by DRAM (the means twice: 2.7 GB for 32 chains of 96^3).  With the component count known to
 // the compiler everything stays in registers and the loads of four chains are in flight together:
-// POOLOLD us with it a variable, POOLNEW so.
+// 677 us with it a variable, 470 us so.
 template <int N>
 __global__ void pool_moments_kernel(const double *mean, const double *m2, long V, int C, double n,
                                     double *mean_aos, double *cov_aos) {

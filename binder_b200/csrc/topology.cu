@@ -250,7 +250,7 @@ __device__ __forceinline__ void add_sums(double (&s)[N], Red *red) {
 
 // topology_correction_3D.cpp:172-245: periodic forward differences, g[(n1*3+n2)][p] =
 // (pos_n1(p + e_n2) - pos_n1(p)) / vs[n1], and the sums of the positions into red.  32-bit indices
-// // (V <= 2^24).  EXACT: every vs is a power of two, so the products with the reciprocals (v0 .. v2) are
+// (V <= 2^24).  EXACT: every vs is a power of two, so the products with the reciprocals (v0 .. v2) are
 // the quotients to the bit.  Bound by DRAM, with the nine FP64 divisions a voxel by those.
 // 160x192x160: 126 us with 64-bit indices, and 71 for the sums in a kernel of their own; now 121
 // together, 85 without the divisions.
